@@ -1,0 +1,138 @@
+// Shared pieces of the exact slice products on the FP16 tensor cores (zone_gram_oz.cu,
+// zone_isqrt_oz.cu): tcgen05 / mbarrier instructions, the K-major operand tile layout, and the
+// balanced base-256 digits of a 54-bit fixed-point number.
+#pragma once
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace oakg {
+
+namespace {
+
+constexpr int kWaitPolls = 1 << 22;  // bound of every mbarrier wait
+// F + kDigitBias has the digits d_p = byte (6 - p) - 128 of F = sum_p d_p 256^(6 - p)
+constexpr unsigned long long kDigitBias = 0x80808080808080ull;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);  // start address
+  d |= (uint64_t)1 << 16;                   // leading byte offset (unused: K fits one swizzle row)
+  d |= (uint64_t)(1024u >> 4) << 32;        // stride byte offset
+  d |= (uint64_t)1 << 46;                   // descriptor version
+  d |= (uint64_t)2 << 61;                   // 128-byte swizzle
+  return d;
+}
+
+// instruction descriptor: D F32, A and B FP16, both K-major, M = 128, N = n
+__device__ __forceinline__ constexpr uint32_t idesc_f16(uint32_t n) {
+  return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                        uint32_t idesc, uint32_t accum) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %3, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %4, p;\n}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(accum), "r"(idesc));
+}
+
+__device__ __forceinline__ void mma_commit(uint32_t mbar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                   mbar)
+               : "memory");
+}
+
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
+  for (int i = 0; i < kWaitPolls; i++) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+__device__ __forceinline__ void fence_before() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void fence_after() {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+// 8 consecutive accumulator columns of this warp's 32 tensor-memory lanes
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// byte offset of the 16-byte chunk `chunk` (8 observations) of operand row `row` in a slice
+__device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
+  return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4));
+}
+
+// The seven digits of two biased fixed-point numbers (F + kDigitBias) as packed FP16 pairs, a in
+// the low half: out[p] holds digit p = byte (6 - p) - 128. 0x6400 | byte is the FP16 number
+// 1024 + byte, and subtracting 1152 is exact: five instructions for two digits of a pair,
+// where a conversion through FP32 takes eighteen.
+__device__ __forceinline__ void digit_pairs(unsigned long long a, unsigned long long b,
+                                            uint32_t (&out)[7]) {
+  const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b,
+                 bh = (uint32_t)(b >> 32);
+  const __half2 bias = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));
+  auto pair = [&](uint32_t m, uint32_t sel) {
+    const uint32_t w = __byte_perm(m, 0x64646464u, sel);
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&w), bias);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  };
+  // bytes 0 (then 1) of a and b side by side, bytes 2 and 3 likewise
+  const uint32_t l01 = __byte_perm(al, bl, 0x5140), l23 = __byte_perm(al, bl, 0x7362);
+  const uint32_t h01 = __byte_perm(ah, bh, 0x5140), h23 = __byte_perm(ah, bh, 0x7362);
+  out[6] = pair(l01, 0x4140);
+  out[5] = pair(l01, 0x4342);
+  out[4] = pair(l23, 0x4140);
+  out[3] = pair(l23, 0x4342);
+  out[2] = pair(h01, 0x4140);
+  out[1] = pair(h01, 0x4342);
+  out[0] = pair(h23, 0x4140);
+}
+
+// vt 2^e2 rounded to nearest even, by integer operations (the conversion and scaling FP64
+// instructions avoided); |vt| < 2^63. Outside FP64's normal range the FP64 operations decide.
+__device__ __forceinline__ double scaled_i64(long long vt, int e2) {
+  if (vt == 0) return 0.0;
+  const unsigned long long sgn = vt < 0 ? (1ull << 63) : 0ull;
+  const unsigned long long m = vt < 0 ? (unsigned long long)(-vt) : (unsigned long long)vt;
+  const int lz = __clzll((long long)m);
+  const int be = 63 - lz + e2 + 1023;
+  if (be < 1 || be > 2045) {
+    int ex = e2 + 1023;
+    ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
+    return (double)vt * __longlong_as_double((long long)ex << 52);
+  }
+  const unsigned long long mm = m << lz;  // leading one at bit 63
+  const unsigned long long mant = (mm >> 11) & 0xFFFFFFFFFFFFFull;
+  const unsigned long long rem = mm & 0x7FFull;
+  const unsigned long long up = (rem > 0x400ull || (rem == 0x400ull && (mant & 1ull))) ? 1ull : 0ull;
+  return __longlong_as_double((long long)(sgn | (((unsigned long long)be << 52) + mant + up)));
+}
+
+}  // namespace
+
+}  // namespace oakg

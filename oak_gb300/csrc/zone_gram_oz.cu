@@ -8,7 +8,7 @@
 // and for every selected observation the FP64 weight w of zone_gram.cu (FP64 distance,
 // exp(-(d/L)^2) or locfun(d/L)). The Gram matrix G = HS_sel^T diag(c) HS_sel (rrsqrt.F90:135,
 // c = w (w / r), DCDCovar of rrsqrt.F90:395) is formed as X^T X with X = diag(|w| / sqrt(r))
-// HS_sel, in FP64, as an exact integer product on the BF16 tensor cores (the slice splitting
+// HS_sel, in FP64, as an exact integer product on the FP16 tensor cores (the slice splitting
 // of Ozaki et al., "Error-free transformations of matrix multiplication by using fast routines
 // of matrix multiplication and its applications", Numer. Algorithms 59 (2012)):
 //
@@ -17,14 +17,14 @@
 //   an integer below 2^54 in magnitude, taken from the FP64 bit pattern with integer
 //   operations. F is written in 7 balanced base-256 digits, F = sum_p d_p 256^(6-p) with
 //   d_0 in [-64, 64] and d_1..d_6 in [-128, 127] (the bytes of F + 0x80808080808080 minus 128);
-//   every digit is exact in BF16.
+//   every digit is exact in FP16.
 //   Then G_ab = 2^(E_a + E_b - 12) sum_L 256^-L level_L(a, b), level_L = sum_{p+q=L} D_p^T D_q
 //   (D_p the digit-p matrix of the zone's rows), for levels 0..6. Levels 7..12 are left out:
 //   a row adds at most 6 x 2^14 x 256^5 = 1.5 x 2^56 to level 7 against 2^108 = F_a F_b at the
 //   column bounds, so they weigh at most ~2^-51.4 of 2^(E_a + E_b) a row when every digit sits
 //   at its bound with one sign (far less for data). A K-tile of 64 observations is staged as
-//   7 digit slices (64 members x 64 observations of BF16, K-major, 128-byte swizzle) and each
-//   K-step of 16 observations issues tcgen05.mma kind::f16 (BF16 x BF16 -> FP32) with
+//   7 digit slices (64 members x 64 observations of FP16, K-major, 128-byte swizzle) and each
+//   K-step of 16 observations issues tcgen05.mma kind::f16 (FP16 x FP16 -> FP32) with
 //   A = [D_p ; D_(p+1)] (M = 128; only rows 0-63 are read back) and B = the run of slices whose
 //   level block lands in the right accumulator column: levels 0..3 in tensor-memory columns
 //   0..255 (4 MMAs a K-step), levels 4..6 in columns 256..447 (7 MMAs a K-step).
@@ -55,6 +55,7 @@
 #include <math.h>
 
 #include "oakg_internal.cuh"
+#include "oz_slices.cuh"
 #include "selection.cuh"
 
 namespace oakg {
@@ -63,18 +64,16 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int NB = 64;                 // padded ensemble width
-constexpr int KT = 64;                 // observations per K-tile (128 bytes of BF16 a row)
+constexpr int KT = 64;                 // observations per K-tile (128 bytes of FP16 a row)
 constexpr int kDigits = 7;
 constexpr int kRing = 1024;            // selected-observation ring (power of two)
 constexpr uint32_t kSliceBytes = 64u * 128u;         // one digit slice of a K-tile
 constexpr uint32_t kBufBytes = kDigits * kSliceBytes;  // one K-tile buffer
 constexpr uint32_t kTmemCols = 512;
-constexpr int kWaitPolls = 1 << 22;
 constexpr int kFlushTiles = 4;         // K-tiles between accumulator reads (256 observations)
 constexpr int kTri = NB * (NB + 1) / 2;
 constexpr int kLevelsExact = 4;        // levels held as 64-bit integer sums
 constexpr int kStageGroups = kThreads / NB;  // threads a member in the staging (8-obs chunks)
-constexpr unsigned long long kDigitBias = 0x80808080808080ull;
 // dynamic shared memory: alignment slack, two K-tile buffers, the slice past the second buffer
 // (rows 64-127 of the A operand of the last digit: read by the MMA, never read back), the
 // integer and FP32 level sums (lower triangle) and the FP64 innovation partials
@@ -102,79 +101,6 @@ struct OzShared {
   sel::ScanRange sr;   // the zone's cell range
   double iL;           // 1 / L
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-// shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);  // start address
-  d |= (uint64_t)1 << 16;                   // leading byte offset (unused: K fits one swizzle row)
-  d |= (uint64_t)(1024u >> 4) << 32;        // stride byte offset
-  d |= (uint64_t)1 << 46;                   // descriptor version
-  d |= (uint64_t)2 << 61;                   // 128-byte swizzle
-  return d;
-}
-
-// instruction descriptor: D F32, A and B BF16, both K-major, M = 128, N = n
-__device__ __forceinline__ uint32_t idesc_bf16(uint32_t n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accum) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %3, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %4, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(accum), "r"(idesc));
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   mbar)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-  for (int i = 0; i < kWaitPolls; i++) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(mbar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-// 8 consecutive accumulator columns of this warp's 32 tensor-memory lanes
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
-  uint32_t r[8];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
-}
-
-// byte offset of the 16-byte chunk `chunk` (8 observations) of operand row `row` in a slice
-__device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
-  return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4));
-}
 
 // round(s h 2^(54 - E)) for s >= 0 (|s h| <= 2^E), from the FP64 bit patterns with integer
 // arithmetic: the product of the two 53-bit significands is exact in 128 bits and rounded once
@@ -214,11 +140,6 @@ __device__ __forceinline__ long long fixed_prod(double s, double h, int E, int& 
     return 0;
   }
   return (hb >> 63) ? -(long long)F : (long long)F;
-}
-
-// BF16 bits of the digit (byte - 128), exact: the FP32 value has at most 8 significant bits
-__device__ __forceinline__ uint32_t digit_bits(uint32_t byte) {
-  return __float_as_uint(__uint_as_float(0x4B3FFF80u + byte) - 12582912.f);
 }
 
 // 64-bit-integer / FP32 lower-triangle index of (row j, column c <= j)
@@ -417,25 +338,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
 #pragma unroll
         for (int i = 0; i < 8; i += 2) {
-          uint32_t lo2[2], hi2[2];
+          unsigned long long U[2];
 #pragma unroll
-          for (int u = 0; u < 2; u++) {
-            const long long F = fixed_prod(sv[i + u], hv[i + u], Ea, bad);
-            const unsigned long long U = (unsigned long long)F + kDigitBias;
-            lo2[u] = (uint32_t)U;
-            hi2[u] = (uint32_t)(U >> 32);
-          }
-          const int wd = i >> 1;
-          // digit p is byte 6 - p of U: p = 0..2 in the high word, 3..6 in the low word
+          for (int u = 0; u < 2; u++)
+            U[u] = (unsigned long long)fixed_prod(sv[i + u], hv[i + u], Ea, bad) + kDigitBias;
+          uint32_t d[kDigits];
+          digit_pairs(U[0], U[1], d);
 #pragma unroll
-          for (int p = 0; p < kDigits; p++) {
-            const int byte = 6 - p;
-            const uint32_t b0 = (byte >= 4) ? (hi2[0] >> (8 * (byte - 4))) & 255u
-                                            : (lo2[0] >> (8 * byte)) & 255u;
-            const uint32_t b1 = (byte >= 4) ? (hi2[1] >> (8 * (byte - 4))) & 255u
-                                            : (lo2[1] >> (8 * byte)) & 255u;
-            pk[p][wd] = __byte_perm(digit_bits(b0), digit_bits(b1), 0x7632);
-          }
+          for (int p = 0; p < kDigits; p++) pk[p][i >> 1] = d[p];
         }
 #pragma unroll
         for (int p = 0; p < kDigits; p++)
@@ -454,17 +364,17 @@ __global__ void __launch_bounds__(kThreads, 1)
           // levels 0..3, columns 64 L: A = [D_p ; D_p+1], B = D_0 .. D_(3-p) into L = p .. 3
 #pragma unroll
           for (int p = 0; p < 4; p++)
-            mma_bf16(tmem + 64 * p, make_desc(base + p * kSliceBytes + ko), make_desc(base + ko),
-                     idesc_bf16(64u * (4 - p)), p == 0 ? acc0 : 1u);
+            mma_f16(tmem + 64 * p, make_desc(base + p * kSliceBytes + ko), make_desc(base + ko),
+                     idesc_f16(64u * (4 - p)), p == 0 ? acc0 : 1u);
           // levels 4..6, columns 256 + 64 (L - 4): B = D_qlo .. D_qhi, q = L - p
 #pragma unroll
           for (int p = 0; p < kDigits; p++) {
             const int qlo = (4 - p > 0) ? 4 - p : 0;
             const int qhi = (6 - p < kDigits - 1) ? 6 - p : kDigits - 1;
             const int off = qlo - (4 - p);
-            mma_bf16(tmem + 256 + 64 * off, make_desc(base + p * kSliceBytes + ko),
+            mma_f16(tmem + 256 + 64 * off, make_desc(base + p * kSliceBytes + ko),
                      make_desc(base + qlo * kSliceBytes + ko),
-                     idesc_bf16(64u * (qhi - qlo + 1)), p == 0 ? acc0 : 1u);
+                     idesc_f16(64u * (qhi - qlo + 1)), p == 0 ? acc0 : 1u);
           }
         }
         mma_commit(mbar0 + 8 * b);
@@ -812,26 +722,6 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// vt 2^e2 rounded to nearest even, by integer operations (the conversion and scaling FP64
-// instructions avoided); |vt| < 2^63. Outside FP64's normal range the FP64 operations decide.
-__device__ __forceinline__ double scaled_i64(long long vt, int e2) {
-  if (vt == 0) return 0.0;
-  const unsigned long long sgn = vt < 0 ? (1ull << 63) : 0ull;
-  const unsigned long long m = vt < 0 ? (unsigned long long)(-vt) : (unsigned long long)vt;
-  const int lz = __clzll((long long)m);
-  const int be = 63 - lz + e2 + 1023;
-  if (be < 1 || be > 2045) {
-    int ex = e2 + 1023;
-    ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
-    return (double)vt * __longlong_as_double((long long)ex << 52);
-  }
-  const unsigned long long mm = m << lz;  // leading one at bit 63
-  const unsigned long long mant = (mm >> 11) & 0xFFFFFFFFFFFFFull;
-  const unsigned long long rem = mm & 0x7FFull;
-  const unsigned long long up = (rem > 0x400ull || (rem == 0x400ull && (mant & 1ull))) ? 1ull : 0ull;
-  return __longlong_as_double((long long)(sgn | (((unsigned long long)be << 52) + mant + up)));
-}
-
 // the seven levels' 8 columns at c0 of this warp's 32 lanes: seven loads, one wait; the empty
 // asm statements tie the registers' uses to the wait
 __device__ __forceinline__ void tmem_ld7x8(uint32_t ta, int c0, uint32_t (&r)[56]) {
@@ -940,24 +830,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t pk[kDigits][4];
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
-      uint32_t lo2[2], hi2[2];
+      unsigned long long Ub[2];
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
-        const long long F = fixed_prod(sv[i + u], hv[i + u], Ea, bad);
-        const unsigned long long Ub = (unsigned long long)F + kDigitBias;
-        lo2[u] = (uint32_t)Ub;
-        hi2[u] = (uint32_t)(Ub >> 32);
-      }
-      const int wd = i >> 1;
+      for (int u = 0; u < 2; u++)
+        Ub[u] = (unsigned long long)fixed_prod(sv[i + u], hv[i + u], Ea, bad) + kDigitBias;
+      uint32_t d[kDigits];
+      digit_pairs(Ub[0], Ub[1], d);
 #pragma unroll
-      for (int p = 0; p < kDigits; p++) {
-        const int byte = 6 - p;
-        const uint32_t b0 = (byte >= 4) ? (hi2[0] >> (8 * (byte - 4))) & 255u
-                                        : (lo2[0] >> (8 * byte)) & 255u;
-        const uint32_t b1 = (byte >= 4) ? (hi2[1] >> (8 * (byte - 4))) & 255u
-                                        : (lo2[1] >> (8 * byte)) & 255u;
-        pk[p][wd] = __byte_perm(digit_bits(b0), digit_bits(b1), 0x7632);
-      }
+      for (int p = 0; p < kDigits; p++) pk[p][i >> 1] = d[p];
     }
 #pragma unroll
     for (int p = 0; p < kDigits; p++)
@@ -976,17 +856,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         // levels 0..3 in columns 64 L: A = [D_p ; D_p+1], B = D_0 .. D_(3-p)
 #pragma unroll
         for (int p = 0; p < 4; p++)
-          mma_bf16(tmem + 64 * p, make_desc(tile_addr + p * kSliceBytes + ko),
-                   make_desc(tile_addr + ko), idesc_bf16(64u * (4 - p)), p == 0 ? acc0 : 1u);
+          mma_f16(tmem + 64 * p, make_desc(tile_addr + p * kSliceBytes + ko),
+                   make_desc(tile_addr + ko), idesc_f16(64u * (4 - p)), p == 0 ? acc0 : 1u);
         // levels 4..6 in columns 256 + 64 (L - 4): B = D_qlo .. D_qhi, q = L - p
 #pragma unroll
         for (int p = 0; p < kDigits; p++) {
           const int qlo = (4 - p > 0) ? 4 - p : 0;
           const int qhi = (6 - p < kDigits - 1) ? 6 - p : kDigits - 1;
           const int off = qlo - (4 - p);
-          mma_bf16(tmem + 256 + 64 * off, make_desc(tile_addr + p * kSliceBytes + ko),
+          mma_f16(tmem + 256 + 64 * off, make_desc(tile_addr + p * kSliceBytes + ko),
                    make_desc(tile_addr + qlo * kSliceBytes + ko),
-                   idesc_bf16(64u * (qhi - qlo + 1)), p == 0 ? acc0 : 1u);
+                   idesc_f16(64u * (qhi - qlo + 1)), p == 0 ? acc0 : 1u);
         }
       }
       mma_commit(mbar);
