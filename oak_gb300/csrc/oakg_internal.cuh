@@ -13,6 +13,7 @@ enum : int32_t {
   ZST_EIG = 2,       // QL iterations did not converge
   ZST_CAPACITY = 4,  // zone larger than the kernel's row tile (cannot happen: tiles split)
   ZST_TIMEOUT = 8,   // a bounded device wait expired (tensor-core pipeline)
+  ZST_RETRY = 16,    // zone left to the FP64 eigensolve (internal to zone_eig_fp64)
 };
 
 // Cell grid over observation coordinates (u, v): cells are cs_u x cs_v, nu x nv of them,
@@ -197,6 +198,15 @@ cudaError_t zone_eig_fp32(int N, int32_t nzc, float* d_GT, const float* d_g,
                           const int32_t* d_nobs, int rotate, float* d_ampl, int32_t* d_status,
                           float* d_aux, float* d_Z, int32_t* d_work, cudaStream_t st);
 size_t zone_eig_aux(int N);
+// ---- zone_isqrt_oz.cu: T = A^(-1/2) Omega and ampl = A^-1 g (A = I + G, G in d_GT, replaced by T)
+// of zones [0, nzc) with nobs > 0, N <= isqrt_oz_max_n(), from FP32 eigenpairs of G: vectors
+// vector-major in d_V (N x N a zone), eigenvalues at d_aux32[3N + k] (zone_eig_aux(N) a zone).
+// Sets each zone's d_status: 0, ZST_NAN, ZST_TIMEOUT, or ZST_RETRY (counted in *d_retries) with G
+// left as it was where the eigenpairs were no start.
+int isqrt_oz_max_n();
+cudaError_t zone_isqrt_oz(int N, int32_t nzc, double* d_GT, const float* d_V, const float* d_aux32,
+                          const double* d_g, const int32_t* d_nobs, int rotate, double* d_ampl,
+                          int32_t* d_status, int32_t* d_retries, cudaStream_t st);
 // zone_eig_fp32 with the FP32 eigenpairs refined to FP64 accuracy (Ogita-Aishima) before T and
 // the amplitudes are formed (zone_refine.cu): d_G0 (N x N floats a zone) keeps G, d_S holds
 // zone_refine_scratch(N) floats a zone; N <= 128.
@@ -213,6 +223,9 @@ cudaError_t zone_eig_refine(int N, int32_t nzc, const float* d_G0, float* d_Z, f
 int eig32_max_n();
 cudaError_t eig32_tridiag(int N, int32_t nzc, float* d_GT, float* d_aux, const int32_t* d_nobs,
                           cudaStream_t st);
+// the same on an FP64 matrix d_G (rounded to FP32, left as it is); the reflectors go to d_GT
+cudaError_t eig32_tridiag_of(int N, int32_t nzc, const double* d_G, float* d_GT, float* d_aux,
+                             const int32_t* d_nobs, cudaStream_t st);
 cudaError_t eig32_values(int N, int32_t nzc, float* d_aux, const int32_t* d_nobs,
                          int32_t* d_status, cudaStream_t st);
 cudaError_t eig32_vectors(int N, int32_t nzc, const float* d_aux, float* d_Z,

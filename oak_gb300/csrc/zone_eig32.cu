@@ -110,8 +110,10 @@ __device__ __forceinline__ float warp_reflector(const float* rowbuf, int k, int 
   return bk;
 }
 
+// src: the matrices (GT itself, or FP64 ones, rounded to FP32).
+template <typename S>
 __global__ void __launch_bounds__(32 * kZpb, 3)
-    k_eig_tridiag32(int N, int32_t nzc, float* __restrict__ GT, float* __restrict__ aux,
+    k_eig_tridiag32(int N, int32_t nzc, const S* src, float* GT, float* __restrict__ aux,
                     const int32_t* __restrict__ nobs) {
   __shared__ __align__(16) float vbuf_s[kZpb][NB];
   __shared__ __align__(16) float wbuf_s[kZpb][NB];
@@ -122,12 +124,13 @@ __global__ void __launch_bounds__(32 * kZpb, 3)
   float* wbuf = wbuf_s[wz];
   float* Gz = GT + (int64_t)zl * N * N;
   float* ax = aux + (int64_t)zl * aux_stride32(N);
+  const S* Sz = src + (int64_t)zl * N * N;
   const int r0 = lane, r1 = lane + 32;
   float a0[NB], a1[NB];
 #pragma unroll
   for (int c = 0; c < NB; c++) {
-    a0[c] = (r0 < N && c < N) ? Gz[r0 * N + c] : 0.f;
-    a1[c] = (r1 < N && c < N) ? Gz[r1 * N + c] : 0.f;
+    a0[c] = (r0 < N && c < N) ? (float)Sz[c * N + r0] : 0.f;  // symmetric: coalesced
+    a1[c] = (r1 < N && c < N) ? (float)Sz[c * N + r1] : 0.f;
   }
   float amax = 0.f;
 #pragma unroll
@@ -358,7 +361,7 @@ __device__ __forceinline__ bool mgs_normalise(int c, int lane, Zone3& zs) {
 }
 
 // mode 0: the whole stage; 1: stop after the back-transform and write the eigenvectors of G
-// (vector-major, over Z); 2: start from eigenvectors of G given in Z (refined, with their
+// (vector-major, over Z; gv is not read); 2: start from eigenvectors of G given in Z (refined, with their
 // eigenvalues in aux) and form T and the amplitudes.
 __global__ void __launch_bounds__(32 * kZpb3, 4)
     k_eig_transform32(int N, int32_t nzc, float* __restrict__ GT, const float* __restrict__ aux,
@@ -385,7 +388,7 @@ __global__ void __launch_bounds__(32 * kZpb3, 4)
     zs.lam[i] = (float)li;
     zs.sq[i] = (float)s;
     zs.qs[i] = (float)sqrt(s);
-    zs.gs[i] = (i < N) ? gv[(int64_t)zl * N + i] : 0.f;
+    zs.gs[i] = (i < N && mode != 1) ? gv[(int64_t)zl * N + i] : 0.f;
     zs.bet[i] = (i < N - 2) ? ax[2 * N + i] : 0.f;
     zs.flag[i] = 1;
   }
@@ -1570,7 +1573,17 @@ cudaError_t eig32_tridiag(int N, int32_t nzc, float* d_GT, float* d_aux, const i
                           cudaStream_t st) {
   if (N < 2 || N > NB) return cudaErrorInvalidValue;
   const int blocks = (nzc + kZpb - 1) / kZpb;
-  k_eig_tridiag32<<<blocks > 0 ? blocks : 1, 32 * kZpb, 0, st>>>(N, nzc, d_GT, d_aux, d_nobs);
+  k_eig_tridiag32<float><<<blocks > 0 ? blocks : 1, 32 * kZpb, 0, st>>>(N, nzc, d_GT, d_GT, d_aux,
+                                                                        d_nobs);
+  return cudaGetLastError();
+}
+
+cudaError_t eig32_tridiag_of(int N, int32_t nzc, const double* d_G, float* d_GT, float* d_aux,
+                             const int32_t* d_nobs, cudaStream_t st) {
+  if (N < 2 || N > NB) return cudaErrorInvalidValue;
+  const int blocks = (nzc + kZpb - 1) / kZpb;
+  k_eig_tridiag32<double><<<blocks > 0 ? blocks : 1, 32 * kZpb, 0, st>>>(N, nzc, d_G, d_GT, d_aux,
+                                                                         d_nobs);
   return cudaGetLastError();
 }
 
