@@ -399,6 +399,14 @@ int run_chunks(Ctx* c, const ChunkArgs& a, int32_t** status_all, double* t_gram,
                                           a.xa32, a.Sa32, *status_all, st)
                          : zone_update_tc(N, zz0, nq, a.zstart, a.xf, a.Sf, a.ldS, T, za, nb,
                                           a.xa, a.Sa, *status_all, st);
+    } else {
+      // plain form: Sa = Sf T on the tensor cores as exact slices, as the Gram
+      const bool sa = a.store32 ? a.Sa32 != nullptr : a.Sa != nullptr;
+      if (!(a.lp.flags & OAKG_FLAG_SIMT_GRAM) && update_oz_pays(N, a.zone_max) && sa)
+        return a.store32 ? zone_update_oz(N, zz0, nq, a.zstart, a.zone_max, a.xf32, a.Sf32, a.ldS,
+                                          T, za, nb, a.xa32, a.Sa32, *status_all, st)
+                         : zone_update_oz(N, zz0, nq, a.zstart, a.zone_max, a.xf, a.Sf, a.ldS, T,
+                                          za, nb, a.xa, a.Sa, *status_all, st);
     }
     return a.store32 ? K::update(N, zz0, nq, a.zstart, a.zone_max, a.xf32, a.Sf32, a.ldS, T, za,
                                  nb, a.xa32, a.Sa32, st)
@@ -1079,8 +1087,12 @@ int analysis_impl(const oakg_dims* dims, const double* xf, const double* Hxf,
   cudaEventRecord(c->ev[3], st);
   if (m == 0) cudaMemsetAsync(d_za, 0, N * sizeof(double), st);
   int32_t zone_max = (int32_t)std::min<int64_t>(n, INT32_MAX);
-  e = zone_update_fp64(N, 0, 1, d_zstart, zone_max, d_xf, d_Sf, ldS, d_G, d_za, d_nobs, d_xa,
-                       d_Sa, st);
+  if (update_oz_pays(N, zone_max) && d_Sa)
+    e = zone_update_oz(N, 0, 1, d_zstart, zone_max, d_xf, d_Sf, ldS, d_G, d_za, d_nobs, d_xa, d_Sa,
+                       d_status, st);
+  else
+    e = zone_update_fp64(N, 0, 1, d_zstart, zone_max, d_xf, d_Sf, ldS, d_G, d_za, d_nobs, d_xa,
+                         d_Sa, st);
   if (e != cudaSuccess) return cuda_fail(e, "update kernel");
   cudaEventRecord(c->ev[4], st);
   if (d_ampl) {

@@ -303,6 +303,22 @@ cudaError_t write_amplitudes_fp32(int N, int32_t z0, int32_t nzc, const float* d
                                   const int32_t* d_nobs, int all_zones, float* ampl_out,
                                   cudaStream_t st);
 
+// Plain form on the tensor cores (zone_update_oz.cu), N <= update_oz_max_n(): zone_update_fp64 with
+// Sa = Sf T as exact slice products; Sa is required; S: double or float storage. d_err receives
+// ZST_TIMEOUT (OR) if a bounded device wait expired.
+int update_oz_max_n();
+// Whether it is the faster one: its cost does not fall with N (padded to 64), the CUDA-core
+// kernel's does with N^2. Zones of 20 rows (16,200): 0.71 ms against 1.40 at N = 64, 0.89 at 52,
+// 0.51 at 40; one zone of 324,000 rows: 0.33 ms against 2.21 at N = 64, 0.49 at 30.
+inline bool update_oz_pays(int N, int32_t zone_max) {
+  return N <= update_oz_max_n() && N >= (zone_max <= 32 ? 47 : 26);
+}
+template <typename S>
+cudaError_t zone_update_oz(int N, int32_t z0, int32_t nzc, const int64_t* d_zone_start,
+                           int32_t zone_max, const S* xf, const S* Sf, int64_t ldS,
+                           const double* d_T, const double* d_ampl, const int32_t* d_nobs, S* xa,
+                           S* Sa, int32_t* d_err, cudaStream_t st);
+
 // Mixed form on the tensor cores (zone_update_tc.cu), N <= 128: the same update with
 // Sa = Sf T and Sf ampl as one 3xTF32 product; d_err receives ZST_TIMEOUT (OR) if a bounded
 // device wait expired.

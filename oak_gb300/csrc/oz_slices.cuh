@@ -12,6 +12,7 @@ namespace {
 
 constexpr int kWaitPolls = 1 << 22;  // bound of every mbarrier wait
 // F + kDigitBias has the digits d_p = byte (6 - p) - 128 of F = sum_p d_p 256^(6 - p)
+constexpr int kDigits = 7;
 constexpr unsigned long long kDigitBias = 0x80808080808080ull;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -131,6 +132,83 @@ __device__ __forceinline__ double scaled_i64(long long vt, int e2) {
   const unsigned long long rem = mm & 0x7FFull;
   const unsigned long long up = (rem > 0x400ull || (rem == 0x400ull && (mant & 1ull))) ? 1ull : 0ull;
   return __longlong_as_double((long long)(sgn | (((unsigned long long)be << 52) + mant + up)));
+}
+
+// 8 consecutive K elements (54-bit fixed point) of an operand row as digit slices
+// of SLICE bytes
+template <uint32_t SLICE>
+__device__ __forceinline__ void stage_digits(const long long (&F)[8], unsigned char* slices,
+                                             uint32_t off) {
+  uint32_t d[4][kDigits];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    digit_pairs((unsigned long long)F[2 * i] + kDigitBias,
+                (unsigned long long)F[2 * i + 1] + kDigitBias, d[i]);
+#pragma unroll
+  for (int p = 0; p < kDigits; p++)
+    *reinterpret_cast<uint4*>(slices + p * SLICE + off) =
+        make_uint4(d[0][p], d[1][p], d[2][p], d[3][p]);
+}
+
+// round(x 2^(B - E)) for |x| < 2^E, B = 54 or 62, by integer operations: the 64-bit conversion
+// instructions run at the FP64 pipe's rate
+template <int B>
+__device__ __forceinline__ long long fixed_of(double x, int E) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)((b >> 52) & 0x7FFu);
+  if (e == 0) return 0;
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  const int s = e - 1075 + B - E;  // x 2^(B - E) = m 2^s
+  unsigned long long F;
+  if (s >= 0)
+    F = m << (s < 10 ? s : 10);
+  else
+    F = s > -55 ? (m + (1ull << (-s - 1))) >> (-s) : 0ull;
+  return (b >> 63) ? -(long long)F : (long long)F;
+}
+
+// This thread's half (even or odd digits of the first operand) of 8 product columns: the
+// levels' sum in units of 2^(E_row + F_col - 60 + SH). Level L's even part lies in column block L
+// (W columns each), its odd part in block L - 1; ta: the first of the columns in block 0, in this
+// warp's lanes.
+template <uint32_t W, int SH>
+__device__ __forceinline__ void read_levels(uint32_t ta, bool odd, long long (&v)[8]) {
+  uint32_t r[64];
+#pragma unroll
+  for (int L = 0; L < 8; L++) {
+    // odd digits: level L is in block L - 1 (level 0 has none; block 0 is read in its place)
+    const uint32_t col = odd ? (L > 0 ? W * (L - 1) : 0u) : W * L;
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r[8 * L]), "=r"(r[8 * L + 1]), "=r"(r[8 * L + 2]), "=r"(r[8 * L + 3]),
+          "=r"(r[8 * L + 4]), "=r"(r[8 * L + 5]), "=r"(r[8 * L + 6]), "=r"(r[8 * L + 7])
+        : "r"(ta + col));
+  }
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int q = 0; q < 64; q += 16)
+    asm volatile(""
+                 : "+r"(r[q]), "+r"(r[q + 1]), "+r"(r[q + 2]), "+r"(r[q + 3]), "+r"(r[q + 4]),
+                   "+r"(r[q + 5]), "+r"(r[q + 6]), "+r"(r[q + 7]), "+r"(r[q + 8]),
+                   "+r"(r[q + 9]), "+r"(r[q + 10]), "+r"(r[q + 11]), "+r"(r[q + 12]),
+                   "+r"(r[q + 13]), "+r"(r[q + 14]), "+r"(r[q + 15])
+                 :
+                 : "memory");
+  // a level sum x is an integer below 2^22: the bits of x + 1.5 2^23 are kB + x
+  constexpr uint32_t kB = 0x4B400000u, kB2 = kB * 257u;
+  auto biased = [](uint32_t x) { return __float_as_uint(__uint_as_float(x) + 12582912.f); };
+#pragma unroll
+  for (int t = 0; t < 8; t++) {
+    const uint32_t x0 = odd ? kB : biased(r[t]);
+    const int32_t a = (int32_t)((x0 << 8) + biased(r[8 + t]) - kB2);
+    const int32_t b = (int32_t)((biased(r[16 + t]) << 8) + biased(r[24 + t]) - kB2);
+    const int32_t c = (int32_t)((biased(r[32 + t]) << 8) + biased(r[40 + t]) - kB2);
+    const int32_t d = (int32_t)((biased(r[48 + t]) << 8) + biased(r[56 + t]) - (kB2 - (128u << SH)));
+    // modulo 2^64; the product's value fits
+    long long u = (long long)c * (256 >> SH) + (long long)(d >> (8 + SH));
+    u = (long long)b * (16777216 >> SH) + u;
+    v[t] = (long long)((unsigned long long)u + ((unsigned long long)((uint32_t)a << (8 - SH)) << 32));
+  }
 }
 
 }  // namespace

@@ -65,7 +65,6 @@ namespace {
 constexpr int kThreads = 512;
 constexpr int NB = 64;                 // padded ensemble width
 constexpr int KT = 64;                 // observations per K-tile (128 bytes of FP16 a row)
-constexpr int kDigits = 7;
 constexpr int kRing = 1024;            // selected-observation ring (power of two)
 constexpr uint32_t kSliceBytes = 64u * 128u;         // one digit slice of a K-tile
 constexpr uint32_t kBufBytes = kDigits * kSliceBytes;  // one K-tile buffer

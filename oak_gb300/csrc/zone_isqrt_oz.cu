@@ -51,7 +51,6 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int NB = 64;  // padded ensemble width
-constexpr int kDigits = 7;
 constexpr uint32_t kSlice = 64u * 128u;
 constexpr uint32_t kTmemCols = 512;
 // dynamic shared memory (1024-aligned): A (7 digit slices and a zero slice), Y (likewise), V
@@ -136,40 +135,7 @@ __device__ __forceinline__ void stage_f16(const float (&x)[8], unsigned char* sl
   *reinterpret_cast<uint4*>(slices + kSlice + off) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// 8 consecutive K elements (54-bit fixed point) of an operand row as digit slices
-__device__ __forceinline__ void stage_digits(const long long (&F)[8], unsigned char* slices,
-                                             uint32_t off) {
-  uint32_t d[4][kDigits];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-    digit_pairs((unsigned long long)F[2 * i] + kDigitBias,
-                (unsigned long long)F[2 * i + 1] + kDigitBias, d[i]);
-#pragma unroll
-  for (int p = 0; p < kDigits; p++)
-    *reinterpret_cast<uint4*>(slices + p * kSlice + off) =
-        make_uint4(d[0][p], d[1][p], d[2][p], d[3][p]);
-}
-
-// The conversions below use integer operations: the 64-bit conversion instructions run at the
-// FP64 pipe's rate.
-
-// round(x 2^(B - E)) for |x| < 2^E, B = 54 or 62
-template <int B>
-__device__ __forceinline__ long long fixed_of(double x, int E) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int e = (int)((b >> 52) & 0x7FFu);
-  if (e == 0) return 0;
-  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
-  const int s = e - 1075 + B - E;  // x 2^(B - E) = m 2^s
-  unsigned long long F;
-  if (s >= 0)
-    F = m << (s < 10 ? s : 10);
-  else
-    F = s > -55 ? (m + (1ull << (-s - 1))) >> (-s) : 0ull;
-  return (b >> 63) ? -(long long)F : (long long)F;
-}
-
-// x 2^sh towards zero, |x 2^sh| < 2^62
+// (by integer operations, as fixed_of in oz_slices.cuh) x 2^sh towards zero, |x 2^sh| < 2^62
 __device__ __forceinline__ long long fixed_of(float x, int sh) {
   const uint32_t b = __float_as_uint(x);
   const int e = (int)((b >> 23) & 255u);
@@ -195,47 +161,6 @@ __device__ __forceinline__ float float_of(double x) {
   if (ae <= 896u) return 0.f;
   return __uint_as_float((hi & 0x80000000u) |
                          ((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29)));
-}
-
-// This thread's half (even or odd digits of the first operand) of 8 product columns: the
-// levels' sum in units of 2^(E_row + F_col - 60). ta: column c0 of block 0 in this warp's lanes.
-__device__ __forceinline__ void read_levels(uint32_t ta, bool odd, long long (&v)[8]) {
-  uint32_t r[64];
-#pragma unroll
-  for (int L = 0; L < 8; L++) {
-    // odd digits: level L is in block L - 1 (level 0 has none; block 0 is read in its place)
-    const uint32_t col = odd ? (L > 0 ? 64u * (L - 1) : 0u) : 64u * L;
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(r[8 * L]), "=r"(r[8 * L + 1]), "=r"(r[8 * L + 2]), "=r"(r[8 * L + 3]),
-          "=r"(r[8 * L + 4]), "=r"(r[8 * L + 5]), "=r"(r[8 * L + 6]), "=r"(r[8 * L + 7])
-        : "r"(ta + col));
-  }
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int q = 0; q < 64; q += 16)
-    asm volatile(""
-                 : "+r"(r[q]), "+r"(r[q + 1]), "+r"(r[q + 2]), "+r"(r[q + 3]), "+r"(r[q + 4]),
-                   "+r"(r[q + 5]), "+r"(r[q + 6]), "+r"(r[q + 7]), "+r"(r[q + 8]),
-                   "+r"(r[q + 9]), "+r"(r[q + 10]), "+r"(r[q + 11]), "+r"(r[q + 12]),
-                   "+r"(r[q + 13]), "+r"(r[q + 14]), "+r"(r[q + 15])
-                 :
-                 : "memory");
-  // a level sum x is an integer below 2^22: the bits of x + 1.5 2^23 are kB + x
-  constexpr uint32_t kB = 0x4B400000u, kB2 = kB * 257u;
-  auto biased = [](uint32_t x) { return __float_as_uint(__uint_as_float(x) + 12582912.f); };
-#pragma unroll
-  for (int t = 0; t < 8; t++) {
-    const uint32_t x0 = odd ? kB : biased(r[t]);
-    const int32_t a = (int32_t)((x0 << 8) + biased(r[8 + t]) - kB2);
-    const int32_t b = (int32_t)((biased(r[16 + t]) << 8) + biased(r[24 + t]) - kB2);
-    const int32_t c = (int32_t)((biased(r[32 + t]) << 8) + biased(r[40 + t]) - kB2);
-    const int32_t d = (int32_t)((biased(r[48 + t]) << 8) + biased(r[56 + t]) - (kB2 - 128u));
-    // modulo 2^64; the product's value fits
-    long long u = (long long)c * 256 + (long long)(d >> 8);
-    u = (long long)b * 16777216 + u;
-    v[t] = (long long)((unsigned long long)u + ((unsigned long long)((uint32_t)a << 8) << 32));
-  }
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -342,10 +267,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   };
   // both halves of the level products: v = the thread's 8 columns of its row
   auto gather_levels = [&](long long (&v)[8]) {
-    read_levels(tlane + 8 * gi_give, odd, v);
+    read_levels<64, 0>(tlane + 8 * gi_give, odd, v);
 #pragma unroll
     for (int t = 0; t < 8; t++) xch[(8 * gi_give + t) * NB + j] = v[t];
-    read_levels(tlane + c0, odd, v);
+    read_levels<64, 0>(tlane + c0, odd, v);
     fence_before();
     __syncthreads();
 #pragma unroll
@@ -484,7 +409,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       long long F[8];
 #pragma unroll
       for (int t = 0; t < 8; t++) F[t] = fixed_of<54>(ga[t], Ei);
-      stage_digits(F, sm + kOffA, own_off);
+      stage_digits<kSlice>(F, sm + kOffA, own_off);
     }
     long long Y[8];
     float esum = 0.f;
@@ -512,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           F[t] = (Y[t] + 32) >> 6;
           Y[t] = F[t] * 64;
         }
-        stage_digits(F, sm + kOffY, own_off);
+        stage_digits<kSlice>(F, sm + kOffY, own_off);
       }
       if ((timeout = !publish())) break;
       if (tid == 0) issue_levels(sa + kOffA, sa + kOffY);  // Z = A Y

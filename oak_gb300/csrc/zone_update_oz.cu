@@ -1,0 +1,302 @@
+// K5 of the plain (FP64) form on the tensor cores, ensembles of up to 64 members:
+//   Sa(i1:i2,:) = Sf(i1:i2,:) T,  xa(i1:i2) = xf(i1:i2) + Sf(i1:i2,:) ampl
+// (rrsqrt.F90:151,165-185,462-464) with the product as exact slices (oz_slices.cuh). T's columns
+// are the first operand ([D_p ; D_(p+1)] of 64 members: M = 128 without padding, staged once a
+// zone), the zone's state rows the second one in tiles of RT rows, so that a short zone costs a
+// short product: Sa^T = T^T Sf^T. Column c of T and row r of Sf get a power of two each (54 bits
+// below their largest element); all levels 0..7 are summed as in zone_isqrt_oz.cu, and an
+// element of Sa is formed in units of 2^(E_c + F_r - 57) and rounded once to FP64. The mean is one
+// FP64 multiply-add an element.
+//
+// RT = 32 (zones of up to 32 rows): 256 threads and 256 tensor-memory columns, two CTAs an SM, one
+// staging while the other multiplies. RT = 64: 512 threads, one CTA an SM, a long zone's tiles
+// spread over several CTAs. Reads and writes are in place safe (a tile is read before it is
+// written; Sa may alias Sf, xa may alias xf). Every mbarrier wait is bounded (ZST_TIMEOUT).
+//
+// Measured, N = 64: 64,800 zones of 20 rows 2.85 ms (9.4 on the FP64 pipe, which its 2 n N^2 flops
+// bind at 1.2 TFLOP/s; 1.33 GB and T's 2.1 GB take 0.5 ms), one zone of 324,000 rows 0.33 ms (2.21).
+// What bounds it: the staging and the read of the levels, which run one after the other in a CTA.
+#include <cuda_runtime.h>
+
+#include "oakg_internal.cuh"
+#include "oz_slices.cuh"
+
+namespace oakg {
+
+namespace {
+
+constexpr uint32_t kSliceT = 64u * 128u;  // a digit slice of T: 64 members
+
+template <int RT>
+struct UpdOz {
+  static constexpr int TT = 8 * RT;                  // threads
+  static constexpr uint32_t kSliceS = RT * 128u;     // a digit slice of RT state rows
+  static constexpr uint32_t kOffS = 8 * kSliceT;     // T: 7 digit slices and a zero slice
+  // the exchange of the two halves' sums overlays the rows' slices
+  static constexpr size_t kRows = 7 * (size_t)kSliceS;
+  static_assert(kRows >= 64 * RT * sizeof(long long), "exchange");
+  static constexpr size_t kSmem = 1024 + kOffS + kRows;
+  static constexpr uint32_t kCols = 8 * RT;          // tensor-memory columns
+};
+
+template <int RT, typename S>
+__global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
+    k_zone_update_oz(int N, int32_t z0, int32_t nzc, int nsplit,
+                     const int64_t* __restrict__ zone_start, const S* xf, const S* Sf, int64_t ldS,
+                     const double* __restrict__ T, const double* __restrict__ ampl,
+                     const int32_t* __restrict__ nobs, S* xa, S* Sa, int32_t* __restrict__ err) {
+  using U = UpdOz<RT>;
+  extern __shared__ __align__(16) unsigned char dyn_raw[];
+  __shared__ __align__(16) double px[8][RT];
+  __shared__ double am[64];
+  __shared__ int32_t emT[64], emS[RT];
+  __shared__ unsigned long long s_mbar;
+  __shared__ uint32_t s_tmem;
+  const uint32_t raw_addr = smem_u32(dyn_raw);
+  const uint32_t pad = ((raw_addr + 1023u) & ~1023u) - raw_addr;
+  unsigned char* sm = dyn_raw + pad;
+  const uint32_t sa = raw_addr + pad;
+  long long* xch = reinterpret_cast<long long*>(sm + U::kOffS);  // [RT rows][64 members]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // tensor-memory lane quarter q: members 32 (q & 1) .. + 31, odd digits for q >= 2; the thread
+  // owns member j, state rows 8 gi .. 8 gi + 7 of the tile
+  const int q = warp & 3, cg = warp >> 2;
+  const bool odd = q >= 2;
+  const int j = 32 * (q & 1) + lane, gi = 2 * cg + (odd ? 1 : 0), gi_give = 2 * cg + (odd ? 0 : 1);
+  const int sr = tid % RT, sc = tid / RT;  // staging: state row, 8-member chunk
+  const uint32_t mbar = smem_u32(&s_mbar);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (uint32_t i = tid; i < kSliceT / 16; i += U::TT)
+    reinterpret_cast<uint4*>(sm + 7 * kSliceT)[i] = make_uint4(0, 0, 0, 0);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&s_tmem)),
+                 "r"(U::kCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = s_tmem;
+  const uint32_t tlane = tmem + ((uint32_t)(32 * q) << 16);
+  uint32_t ph = 0;
+  bool late = false, timeout = false;
+
+  const int64_t items = (int64_t)nzc * nsplit;
+  for (int64_t it = blockIdx.x; it < items && !timeout; it += gridDim.x) {
+    const int32_t zl = (int32_t)(it / nsplit);
+    const int part = (int)(it - (int64_t)zl * nsplit);
+    const int64_t i1 = zone_start[z0 + zl], i2 = zone_start[z0 + zl + 1];
+    // the part's tiles of RT rows
+    const int64_t tiles = (i2 - i1 + RT - 1) / RT;
+    const int64_t t0 = tiles * part / nsplit, t1 = tiles * (part + 1) / nsplit;
+    if (t0 >= t1) continue;  // uniform
+    if (nobs[zl] == 0) {
+      const int64_t r0 = i1 + t0 * RT, r1 = min(i1 + t1 * RT, i2);
+      for (int64_t r = r0 + tid; r < r1; r += U::TT) xa[r] = xf[r];
+      if (Sa != Sf)
+        for (int k = 0; k < N; k++)
+          for (int64_t r = r0 + tid; r < r1; r += U::TT)
+            Sa[r + (int64_t)k * ldS] = Sf[r + (int64_t)k * ldS];
+      continue;
+    }
+    // T: unit (member column c, chunk of 8 k), k along the operand row; the first tile's rows beside
+    constexpr int NU = 512 / U::TT;
+    double tv[NU][8], sv[8];
+    const double* Tz = T + (int64_t)zl * N * N;
+#pragma unroll
+    for (int u = 0; u < NU; u++) {
+      const int c = (tid + u * U::TT) & 63, ch = (tid + u * U::TT) >> 6;
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        const int k = 8 * ch + t;
+        tv[u][t] = (k < N && c < N) ? Tz[(int64_t)k * N + c] : 0.0;
+      }
+    }
+    auto load_rows = [&](int64_t tile) {
+      const int64_t r = i1 + tile * RT + sr;
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        const int k = 8 * sc + t;
+        sv[t] = (r < i2 && k < N) ? (double)Sf[r + (int64_t)k * ldS] : 0.0;
+      }
+    };
+    load_rows(t0);
+    __syncthreads();  // the previous item's shared values are consumed
+    if (tid < 64) {
+      emT[tid] = 0;
+      am[tid] = (tid < N) ? ampl[(int64_t)zl * N + tid] : 0.0;
+    }
+    if (tid < RT) emS[tid] = 0;
+    __syncthreads();
+    auto top = [](const double (&x)[8]) {
+      int e = 0;
+#pragma unroll
+      for (int t = 0; t < 8; t++)
+        e = max(e, (int)(((unsigned long long)__double_as_longlong(x[t]) >> 52) & 0x7FFu));
+      return e;
+    };
+#pragma unroll
+    for (int u = 0; u < NU; u++) atomicMax(&emT[(tid + u * U::TT) & 63], top(tv[u]));
+    for (int64_t tile = t0; tile < t1; tile++) {
+      atomicMax(&emS[sr], top(sv));
+      double x = 0.0;
+#pragma unroll
+      for (int t = 0; t < 8; t++) x = fma(sv[t], am[8 * sc + t], x);
+      px[sc][sr] = x;
+      __syncthreads();  // exponents and partial sums complete
+      if (tile == t0) {
+#pragma unroll
+        for (int u = 0; u < NU; u++) {
+          const int c = (tid + u * U::TT) & 63, ch = (tid + u * U::TT) >> 6;
+          long long F[8];
+#pragma unroll
+          for (int t = 0; t < 8; t++) F[t] = fixed_of<54>(tv[u][t], emT[c] - 1022);
+          stage_digits<kSliceT>(F, sm, tile_off(c, ch));
+        }
+      }
+      {
+        long long F[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) F[t] = fixed_of<54>(sv[t], emS[sr] - 1022);
+        stage_digits<U::kSliceS>(F, sm + U::kOffS, tile_off(sr, sc));
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      fence_before();
+      if (__syncthreads_or(late)) {
+        timeout = true;
+        break;
+      }
+      if (tid == 0) {
+        fence_after();
+        const uint32_t B = sa + U::kOffS;
+#pragma unroll 1
+        for (int kk = 0; kk < 4; kk++) {
+          const uint32_t ko = kk * 32, acc = kk > 0 ? 1u : 0u;
+          const uint64_t b0 = make_desc(B + ko);
+          // D_p D_q, p even (odd in the upper half), in column block p + q
+          uint64_t a = make_desc(sa + ko);
+          if (RT == 32) {
+            mma_f16(tmem, a, b0, idesc_f16(7 * RT), acc);                       // p = 0, q = 0..6
+            a = make_desc(sa + 2 * kSliceT + ko);
+            mma_f16(tmem + 2 * RT, a, b0, idesc_f16(5 * RT), 1u);               // p = 2, q = 0..4
+          } else {
+            mma_f16(tmem, a, b0, idesc_f16(4 * RT), acc);                       // p = 0, q = 0..3
+            mma_f16(tmem + 4 * RT, a, make_desc(B + 4 * U::kSliceS + ko), idesc_f16(3 * RT), acc);
+            a = make_desc(sa + 2 * kSliceT + ko);
+            mma_f16(tmem + 2 * RT, a, b0, idesc_f16(4 * RT), 1u);               // p = 2, q = 0..3
+            mma_f16(tmem + 6 * RT, a, make_desc(B + 4 * U::kSliceS + ko), idesc_f16(RT), 1u);
+          }
+          mma_f16(tmem + 7 * RT, a, make_desc(B + 5 * U::kSliceS + ko), idesc_f16(RT), acc);
+          mma_f16(tmem + 4 * RT, make_desc(sa + 4 * kSliceT + ko), b0, idesc_f16(4 * RT), 1u);
+          mma_f16(tmem + 6 * RT, make_desc(sa + 6 * kSliceT + ko), b0, idesc_f16(2 * RT), 1u);
+        }
+        mma_commit(mbar);
+      }
+      // beside the product: the mean, and the next tile's rows
+      const int64_t rt = i1 + tile * RT;
+      if (tid < RT && rt + tid < i2) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) s += px[k][tid];
+        xa[rt + tid] = (S)((double)xf[rt + tid] + s);
+      }
+      if (tile + 1 < t1) load_rows(tile + 1);
+      if (!mbar_wait(mbar, ph)) late = true;
+      ph ^= 1u;
+      fence_after();
+      long long v[8];
+      read_levels<RT, 3>(tlane + 8 * gi_give, odd, v);
+#pragma unroll
+      for (int t = 0; t < 8; t++) xch[(8 * gi_give + t) * 64 + j] = v[t];
+      read_levels<RT, 3>(tlane + 8 * gi, odd, v);
+      fence_before();
+      __syncthreads();  // halves exchanged; tensor memory read
+      if (j < N) {
+        const bool cbad = emT[j] == 0x7FF;
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const int r = 8 * gi + t;
+          if (rt + r < i2) {
+            double y = scaled_i64(v[t] + xch[r * 64 + j], emT[j] + emS[r] - 2 * 1022 - 57);
+            if (cbad || emS[r] == 0x7FF) y = __longlong_as_double(0x7FF8000000000000ll);
+            Sa[rt + r + (int64_t)j * ldS] = (S)y;
+          }
+        }
+      }
+      __syncthreads();  // the exchange and the exponents are read
+      if (tid < RT) emS[tid] = 0;
+      __syncthreads();
+    }
+  }
+  // teardown: no MMA may still write tensor memory when it is freed
+  if (__syncthreads_or(late) && tid == 0) {
+    atomicOr(err, ZST_TIMEOUT);
+    mbar_wait(mbar, ph ^ 1u);
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(U::kCols));
+}
+
+template <int RT, typename S>
+cudaError_t launch(int N, int32_t z0, int32_t nzc, const int64_t* d_zone_start, int32_t zone_max,
+                   const S* xf, const S* Sf, int64_t ldS, const double* d_T, const double* d_ampl,
+                   const int32_t* d_nobs, S* xa, S* Sa, int32_t* d_err, cudaStream_t st) {
+  using U = UpdOz<RT>;
+  cudaError_t e = cudaFuncSetAttribute(
+      k_zone_update_oz<RT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)U::kSmem);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_zone_update_oz<RT, S>,
+                           cudaFuncAttributePreferredSharedMemoryCarveout,
+                           (int)cudaSharedmemCarveoutMaxShared);
+  if (e != cudaSuccess) return e;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t grid_max = (int64_t)sms * (RT == 32 ? 2 : 1);
+  // a long zone's tiles over several CTAs where the zones alone do not fill the chip
+  const int64_t tiles = (zone_max + RT - 1) / RT;
+  int64_t nsplit = (grid_max + nzc - 1) / nzc;
+  nsplit = nsplit < 1 ? 1 : (nsplit > tiles ? (tiles < 1 ? 1 : tiles) : nsplit);
+  const int64_t items = (int64_t)nzc * nsplit;
+  const int grid = (int)(items < grid_max ? items : grid_max);
+  k_zone_update_oz<RT, S><<<grid, U::TT, U::kSmem, st>>>(N, z0, nzc, (int)nsplit, d_zone_start, xf,
+                                                         Sf, ldS, d_T, d_ampl, d_nobs, xa, Sa, d_err);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+int update_oz_max_n() { return 64; }
+
+template <typename S>
+cudaError_t zone_update_oz(int N, int32_t z0, int32_t nzc, const int64_t* d_zone_start,
+                           int32_t zone_max, const S* xf, const S* Sf, int64_t ldS,
+                           const double* d_T, const double* d_ampl, const int32_t* d_nobs, S* xa,
+                           S* Sa, int32_t* d_err, cudaStream_t st) {
+  if (N < 1 || N > update_oz_max_n() || !Sa) return cudaErrorInvalidValue;
+  if (nzc <= 0) return cudaSuccess;
+  return zone_max <= 32 ? launch<32, S>(N, z0, nzc, d_zone_start, zone_max, xf, Sf, ldS, d_T, d_ampl,
+                                        d_nobs, xa, Sa, d_err, st)
+                        : launch<64, S>(N, z0, nzc, d_zone_start, zone_max, xf, Sf, ldS, d_T, d_ampl,
+                                        d_nobs, xa, Sa, d_err, st);
+}
+
+template cudaError_t zone_update_oz<double>(int, int32_t, int32_t, const int64_t*, int32_t,
+                                            const double*, const double*, int64_t, const double*,
+                                            const double*, const int32_t*, double*, double*,
+                                            int32_t*, cudaStream_t);
+template cudaError_t zone_update_oz<float>(int, int32_t, int32_t, const int64_t*, int32_t,
+                                           const float*, const float*, int64_t, const double*,
+                                           const double*, const int32_t*, float*, float*, int32_t*,
+                                           cudaStream_t);
+
+}  // namespace oakg
