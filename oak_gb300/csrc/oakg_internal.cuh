@@ -110,7 +110,8 @@ cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int 
                          int32_t z0, int32_t nzc, const double* zone_xyzt, const double* corr_len,
                          const double* max_len, double* d_G, double* d_g, int32_t* d_nobs,
                          int brute, int32_t* d_work, int32_t* d_err, void* d_scratch,
-                         cudaStream_t st, const int32_t* order = nullptr);
+                         cudaStream_t st, const int32_t* order = nullptr,
+                         const int32_t* zlist = nullptr);  // zlist: as zone_gram_fp64_list
 // FP32 copy of count doubles (HS rows for the mixed form).
 cudaError_t rows_to_fp32(const double* src, float* dst, int64_t count, cudaStream_t st);
 // FP64 copy of count floats (observation vectors given in FP32 storage).

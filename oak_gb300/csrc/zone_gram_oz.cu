@@ -19,37 +19,47 @@
 //   d_0 in [-64, 64] and d_1..d_6 in [-128, 127] (the bytes of F + 0x80808080808080 minus 128);
 //   every digit is exact in FP16.
 //   Then G_ab = 2^(E_a + E_b - 12) sum_L 256^-L level_L(a, b), level_L = sum_{p+q=L} D_p^T D_q
-//   (D_p the digit-p matrix of the zone's rows), for levels 0..6. Levels 7..12 are left out:
-//   a row adds at most 6 x 2^14 x 256^5 = 1.5 x 2^56 to level 7 against 2^108 = F_a F_b at the
-//   column bounds, so they weigh at most ~2^-51.4 of 2^(E_a + E_b) a row when every digit sits
-//   at its bound with one sign (far less for data). A K-tile of 64 observations is staged as
-//   7 digit slices (64 members x 64 observations of FP16, K-major, 128-byte swizzle) and each
-//   K-step of 16 observations issues tcgen05.mma kind::f16 (FP16 x FP16 -> FP32) with
-//   A = [D_p ; D_(p+1)] (M = 128; only rows 0-63 are read back) and B = the run of slices whose
-//   level block lands in the right accumulator column: levels 0..3 in tensor-memory columns
-//   0..255 (4 MMAs a K-step), levels 4..6 in columns 256..447 (7 MMAs a K-step).
-//   Exactness: a digit product is at most 2^14 (2^13 with d_0), so the FP32 sums of levels 0..3
-//   stay exact integers below 2^24 over 256 observations; the accumulators are read every 4
-//   K-tiles and added into 64-bit integer sums (levels 0..3) and an FP32 sum of
-//   level_4 + level_5 / 256 + level_6 / 65536 (its FP32 rounding, about an ulp of level 4 per
-//   read, weighs ~2^-52 of 2^(E_a + E_b) per 256 observations). At the end of the zone
-//   G = 2^(E_a + E_b - 36) (v + V456 / 256) with v = ((L0 256 + L1) 256 + L2) 256 + L3 as a
-//   64-bit integer, converted once to FP64. The error of G is therefore the rounding of X to
-//   the fixed point (2^-54 of its column scale) and the dropped levels, not the length of the
-//   sums: at most ~2^-51 of 2^(E_a + E_b) per term, typically near 2^-53 (the CPU model of
-//   these steps, tests/test_slice_products_model.py, checks the bound and the budgets).
+//   (D_p the digit-p matrix of the zone's rows), for levels 0..7. Levels 8..12 are left out: a
+//   row adds at most 5 x 2^14 x 256^4 = 1.25 x 2^48 to level 8 against 2^108 = F_a F_b at the
+//   column bounds, 2^-59.7 of 2^(E_a + E_b).
+//   A K-tile of 64 observations is staged as 7 digit slices (64 members x 64 observations of
+//   FP16, K-major, 128-byte swizzle), the buffer's eighth slice is zero (D_7), and each K-step of
+//   16 observations issues tcgen05.mma kind::f16 (FP16 x FP16 -> FP32) with A = [D_p ; D_(p+1)]
+//   (M = 128), p = 0, 2, 4, 6, and B = D_0 .. D_(7-p) into the column blocks p .. 7: block L then
+//   holds level L's products with even p in lanes 0-63 and level L + 1's with odd p in lanes
+//   64-127. Both halves of every MMA are used: 20 block columns a K-step, 7 MMAs of up to 256.
+//   Exactness: a digit product is at most 2^14 (2^13 with d_0) and a half sums at most 4 a row,
+//   so the FP32 sums stay exact integers up to 2^24 over 256 observations; the accumulators are
+//   read every 4 K-tiles and added into two 64-bit integer sums, levels 0..3 and levels 4..7 (in
+//   units of level 6: level 7 is rounded there, 2^-60 of 2^(E_a + E_b) a read). At the end of
+//   the zone G = 2^(E_a + E_b - 36) v_hi + 2^(E_a + E_b - 60) v_lo, each converted once to FP64.
+//   The error of G is therefore the rounding of X to the fixed point (2^-54 of its column scale)
+//   and the last addition, not the length of the sums (the CPU model of these steps,
+//   tests/test_slice_products_model.py, checks the bound and the budgets of the scheme that
+//   stops one level earlier).
 //
 // The innovation projection g = X^T (sqrt(c) d) (rrsqrt.F90:142) is accumulated in FP64 by the
 // staging threads (one FMA per staged element).
 //
-// Pipeline per CTA (one zone at a time, one CTA of 512 threads per SM: its shared memory and
-// the 512 tensor-memory columns admit no second one): candidates are tested 512 at a time
-// (a zone's cell-row ranges flattened into one index space);
-// selected observations go to a ring, their FP64 weights are computed one thread an entry
-// (|w| / sqrt(r) and w^2 / r (yo - Hxf)); every full K-tile is
-// staged into one of two shared buffers (7 slices) and handed to the tensor core by one thread
-// (44 MMAs and a commit to the buffer's mbarrier), so staging of the next tile overlaps the
-// MMAs. Every mbarrier wait is bounded; on expiry the kernel records ZST_TIMEOUT, stops taking
+// What bounds it: the worker warps' integer work and FP64 pipe, in turn with each other, not
+// the tensor cores (busy under 15% of the time) and not memory. The CTA (one per SM: its shared
+// memory and the 512 tensor-memory columns admit no second one) is split by role:
+//   16 worker warps   candidates are tested 512 at a time (a zone's cell-row ranges flattened
+//                     into one index space); selected observations go to a ring, their FP64
+//                     weights are computed one thread an entry (|w| / sqrt(r) as significand and
+//                     exponent, so that staging is one 64 x 64-bit integer product a value;
+//                     w^2 / r (yo - Hxf)); full K-tiles are staged into two shared buffers;
+//   the issuer warp   waits for a staged buffer, issues its 28 MMAs and the commit, so no worker
+//                     spends its time on descriptors;
+//   the scout warp    takes the next zone from the counter and evaluates its FP64 set-up
+//                     (projection, length scales, cell range) while the workers are at this one.
+// Measured on 64,800 zones of a 360 x 180 global grid, N = 50, 3,000 observations, against the
+// same kernel with levels 0..6 in 44 MMAs of which half of each was unused, issued by a worker,
+// the set-up in line and the FP64 multiply-and-split staging: 24.5 ms before, 20.9 ms now; 7,200
+// zones with N = 64: 2.55 ms before, 2.13 ms now. Of about 95,000 cycles a zone 28,000 are staging, 25,000
+// accumulator reads, 24,000 selection and ranges, 10,000 FP64 weights. Reading the accumulators
+// every 8 K-tiles instead of 4 measured the same.
+// Every mbarrier wait is bounded; on expiry the kernel records ZST_TIMEOUT, stops taking
 // zones, waits (bounded) for its MMAs and frees its tensor memory.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -67,24 +77,34 @@ constexpr int NB = 64;                 // padded ensemble width
 constexpr int KT = 64;                 // observations per K-tile (128 bytes of FP16 a row)
 constexpr int kRing = 1024;            // selected-observation ring (power of two)
 constexpr uint32_t kSliceBytes = 64u * 128u;         // one digit slice of a K-tile
-constexpr uint32_t kBufBytes = kDigits * kSliceBytes;  // one K-tile buffer
+constexpr uint32_t kBufBytes = 8 * kSliceBytes;  // one K-tile buffer: the digits and a zero slice
 constexpr uint32_t kTmemCols = 512;
 constexpr int kFlushTiles = 4;         // K-tiles between accumulator reads (256 observations)
 constexpr int kTri = NB * (NB + 1) / 2;
-constexpr int kLevelsExact = 4;        // levels held as 64-bit integer sums
+constexpr int kLdG = NB + 1;
 constexpr int kStageGroups = kThreads / NB;  // threads a member in the staging (8-obs chunks)
-// dynamic shared memory: alignment slack, two K-tile buffers, the slice past the second buffer
-// (rows 64-127 of the A operand of the last digit: read by the MMA, never read back), the
-// integer and FP32 level sums (lower triangle) and the FP64 innovation partials
-constexpr size_t kDynSmem = 1024 + 2 * (size_t)kBufBytes + kSliceBytes +
-                            (size_t)kLevelsExact * kTri * sizeof(long long) +
-                            (size_t)kTri * sizeof(float) + kStageGroups * NB * sizeof(double);
+static_assert(KT == 8 * kStageGroups, "a chunk of 8 observations a thread");
+// dynamic shared memory: alignment slack, two K-tile buffers, the integer level sums (lower
+// triangle) and the FP64 innovation partials
+constexpr size_t kDynSmem = 1024 + 2 * (size_t)kBufBytes + 2 * (size_t)kTri * sizeof(long long) +
+                            kStageGroups * NB * sizeof(double);
+
+// a zone's set-up, by the scout warp
+struct OzZone {
+  double zu, zv, L, Rmax, iL;
+  sel::ZoneCell32 zc;  // the zone's cell-relative FP32 coordinates (read by broadcast)
+  sel::ScanRange sr;   // the zone's cell range
+  int32_t w, zl, z;
+};
 
 struct OzShared {
   int32_t ring_q[kRing];
-  double ring_s[kRing];  // |w| / sqrt(r_q)
+  unsigned long long ring_m[kRing];  // |w| / sqrt(r_q): significand << 11 (0 for a zero)
+  int32_t ring_e[kRing];             // and its biased exponent
   double ring_t[kRing];  // w^2 / r_q (yo - Hxf)_q
-  unsigned long long mbar[2];
+  OzZone zone[2];
+  unsigned long long done[2], full[2];  // a buffer's MMAs complete; its tile staged
+  int32_t first[2];                     // the buffer's tile starts the accumulators
   int32_t warp_cnt[kThreads / 32];
   int32_t rlo[kThreads];   // first observation of each candidate range of a block of ranges
   int32_t roff[kThreads];  // exclusive prefix of the ranges' lengths
@@ -92,13 +112,7 @@ struct OzShared {
   int32_t rtotal;
   int32_t E[NB];         // column exponents
   uint32_t tmem_base;
-  int32_t zone;
-  int32_t nrel;
-  int32_t flag;
-  int32_t bad;
-  sel::ZoneCell32 zc;  // the zone's cell-relative FP32 coordinates (read by broadcast)
-  sel::ScanRange sr;   // the zone's cell range
-  double iL;           // 1 / L
+  int32_t nrel, bad, stop;
 };
 
 // round(s h 2^(54 - E)) for s >= 0 (|s h| <= 2^E), from the FP64 bit patterns with integer
@@ -141,478 +155,589 @@ __device__ __forceinline__ long long fixed_prod(double s, double h, int E, int& 
   return (hb >> 63) ? -(long long)F : (long long)F;
 }
 
-// 64-bit-integer / FP32 lower-triangle index of (row j, column c <= j)
+// round(s h 2^(54 - E)) for s = m 2^(es - 1086) >= 0 (m its significand << 11): the upper 64 of the
+// product's 106 bits are shifted to the fixed point once (the bits below weigh 2^-9 of its unit).
+// The observation's half of the work is done once for all members: 28 integer instructions an
+// element where fixed_prod takes 60.
+__device__ __forceinline__ long long fixed_row(unsigned long long m, int es, double h, int E,
+                                               int& bad) {
+  const unsigned long long hb = (unsigned long long)__double_as_longlong(h);
+  const int eh = (int)(hb >> 52) & 0x7FF;
+  const unsigned long long mh = ((hb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 10;
+  // s h 2^(54 - E) = P 2^-(2096 + E - es - eh), P = (m >> 11) (mh >> 10); top = P >> 43
+  const int r = 2053 + E - es - eh;
+  if (eh == 0x7FF || (r < 7 && m != 0ull && eh != 0)) {  // non-finite, or above the bound
+    bad = 1;
+    return 0;
+  }
+  const unsigned long long top = __umul64hi(m, mh);
+  const unsigned long long F = (r < 64 && eh != 0) ? (top + (1ull << (r - 1))) >> r : 0ull;
+  return (hb >> 63) ? -(long long)F : (long long)F;
+}
+
+// 64-bit-integer lower-triangle index of (row j, column c <= j)
 __device__ __forceinline__ int tri(int j) { return j * (j + 1) / 2; }
 
-__global__ void __launch_bounds__(kThreads, 1)
+// barrier of the worker warps; with the scout warp
+__device__ __forceinline__ void bar_workers() {
+  asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+}
+__device__ __forceinline__ void bar_zone() {
+  asm volatile("bar.sync 2, %0;" ::"n"(kThreads + 32) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+
+__global__ void __launch_bounds__(kThreads + 64, 1)
     k_zone_gram_oz(CellGrid g, SortedObs so, int N, LocParams lp, int32_t z0, int32_t nzc,
                    const double* __restrict__ zone_xyzt, const double* __restrict__ corr_len,
                    const double* __restrict__ max_len, const int32_t* __restrict__ col_exp,
                    const double* __restrict__ isr, double* __restrict__ G,
-                   double* __restrict__ gv, int32_t* __restrict__ nobs, int brute, int32_t* __restrict__ work, int32_t* __restrict__ err,
-                   const int32_t* __restrict__ order) {
+                   double* __restrict__ gv, int32_t* __restrict__ nobs, int brute,
+                   int32_t* __restrict__ work, int32_t* __restrict__ err,
+                   const int32_t* __restrict__ order, const int32_t* __restrict__ zlist) {
   extern __shared__ __align__(16) unsigned char dyn_raw[];
   __shared__ __align__(16) OzShared ts;
   const uint32_t raw_addr = smem_u32(dyn_raw);
   const uint32_t pad = ((raw_addr + 1023u) & ~1023u) - raw_addr;
-  unsigned char* tiles = dyn_raw + pad;  // 2 x kBufBytes + one slice, 1024-aligned
+  unsigned char* tiles = dyn_raw + pad;  // 2 x kBufBytes (7 slices and a zero slice), 1024-aligned
   const uint32_t tile_addr = raw_addr + pad;
-  long long* acc64 = reinterpret_cast<long long*>(tiles + 2 * kBufBytes + kSliceBytes);
-  float* accf = reinterpret_cast<float*>(acc64 + kLevelsExact * kTri);
-  double* gpart = reinterpret_cast<double*>(accf + kTri);  // [kStageGroups][NB]
+  long long* acc_hi = reinterpret_cast<long long*>(tiles + 2 * kBufBytes);  // levels 0..3
+  long long* acc_lo = acc_hi + kTri;                                       // levels 4..7
+  double* gpart = reinterpret_cast<double*>(acc_lo + kTri);  // [kStageGroups][NB]
+  // the halves' exchange overlays the K-tile buffers' digits (free at a read): [64 columns][64 rows]
+  // of levels 0..3 in the first, of levels 4..7 in the second
+  long long* xch = reinterpret_cast<long long*>(tiles);
+  long long* xcl = reinterpret_cast<long long*>(tiles + kBufBytes);
+  double* Gs = reinterpret_cast<double*>(tiles);  // and then the zone's G, [64][kLdG]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // staging: member a, 8-observation chunk kq of a K-tile
-  const int a = tid & (NB - 1), kq = tid >> 6;
-  const uint32_t mbar0 = smem_u32(&ts.mbar[0]);
-
+  const uint32_t done0 = smem_u32(&ts.done[0]), full0 = smem_u32(&ts.full[0]);
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar0));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar0 + 8));
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(done0 + 8 * b));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full0 + 8 * b),
+                   "n"(kThreads / 32));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    ts.flag = 0;
+    ts.stop = 0;
   }
   if (tid < NB) ts.E[tid] = (tid < N) ? col_exp[tid] : 0;
-  // the slice past the second buffer is only read into accumulator rows that are never read
-  // back; it is cleared once so that those rows hold finite values
-  for (uint32_t i = tid; i < kSliceBytes / 16; i += kThreads)
-    reinterpret_cast<uint4*>(tiles + 2 * kBufBytes)[i] = make_uint4(0, 0, 0, 0);
+  // the zero slices past the digits
+  for (uint32_t i = tid; i < 2 * kSliceBytes / 16; i += kThreads + 64)
+    reinterpret_cast<uint4*>(tiles + (i / (kSliceBytes / 16)) * kBufBytes + 7 * kSliceBytes)
+        [i % (kSliceBytes / 16)] = make_uint4(0, 0, 0, 0);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&ts.tmem_base)),
                  "r"(kTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = ts.tmem_base;
-  const int Ea = ts.E[a];
-
   const int64_t ncells = (int64_t)g.nu * g.nv;
   const int full_scan = brute || !lp.localise;
-  const bool fast = (lp.loctype != 1) || (lp.metric == OAKG_METRIC_CARTESIAN);
-  int pend0 = 0, pend1 = 0;   // buffer has MMAs not yet waited for (uniform)
-  uint32_t ph0 = 0, ph1 = 0;  // parity of the buffer's next completion (uniform)
-  bool abort = false;
+  bool late = false;  // a bounded wait of this thread expired
 
-  // wait for buffer b's outstanding MMAs (thread 0, bounded); result published in ts.flag
-  auto drain = [&](int b) {
-    if (tid == 0) {
-      const uint32_t ph = b ? ph1 : ph0;
-      if (!mbar_wait(mbar0 + 8 * b, ph)) ts.flag = 1;
-    }
-    if (b) {
-      ph1 ^= 1u;
-      pend1 = 0;
-    } else {
-      ph0 ^= 1u;
-      pend0 = 0;
-    }
-  };
-
-  // add the accumulators into the level sums (all MMAs complete and published by a barrier).
-  // Warp w reads lanes 32 (w % 4) .. + 31, i.e. rows j of the lower (D_p) half for w % 4 < 2;
-  // warp group h = w / 4 takes levels 2h, 2h + 1 (h < 2) or 4..6 (h = 2); row j keeps columns
-  // c <= j.
-  auto flush = [&]() {
-    fence_after();
-    const int q = warp & 3, h = warp >> 2;
-    if (q < 2 && h < 3) {
-      const int j = 32 * q + lane;
-      const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16);
-      const int ncol = 32 * (q + 1);  // warp-uniform bound of the row's lower triangle
-      const int tj = tri(j);
-      if (h < 2) {
-#pragma unroll
-        for (int L = 2 * h; L < 2 * h + 2; L++) {
-          long long* accL = acc64 + L * kTri + tj;
-          for (int c0 = 0; c0 < ncol; c0 += 8) {
-            float v[8];
-            tmem_ld8(ta + 64 * L + c0, v);
-#pragma unroll
-            for (int t = 0; t < 8; t++)
-              if (c0 + t <= j) accL[c0 + t] += (long long)__float2int_rn(v[t]);
-          }
+  if (warp == kThreads / 32) {
+    // ---- issuer: every complete K-tile to the tensor core, so that no staging warp waits for the
+    // tensor core's queue (28 MMAs a tile: p = 0, 2, 4, 6, [D_p ; D_(p+1)] by D_0 .. D_(7-p))
+    if (lane == 0) {
+      uint32_t phf[2] = {0u, 0u};
+      for (uint32_t n = 0;; n++) {
+        const uint32_t b = n & 1u;
+        if (!mbar_wait(full0 + 8 * b, phf[b])) {
+          late = true;
+          break;
         }
-      } else {
-        float* af = accf + tj;
-        for (int c0 = 0; c0 < ncol; c0 += 8) {
-          float v4[8], v5[8], v6[8];
-          tmem_ld8(ta + 256 + c0, v4);
-          tmem_ld8(ta + 320 + c0, v5);
-          tmem_ld8(ta + 384 + c0, v6);
-#pragma unroll
-          for (int t = 0; t < 8; t++)
-            if (c0 + t <= j) af[c0 + t] += fmaf(v6[t], 1.f / 65536.f, fmaf(v5[t], 1.f / 256.f, v4[t]));
-        }
-      }
-    }
-    fence_before();
-    __syncthreads();
-  };
-
-  for (;;) {
-    if (tid == 0) ts.zone = atomicAdd(work, 1);
-    __syncthreads();
-    const int32_t w = ts.zone;  // pick number; zone order[z0 + w] when a pick order is given
-    if (w >= nzc || ts.flag) break;
-    const int32_t zl = order ? order[z0 + w] : w;
-    const int32_t z = z0 + zl;
-    const double zx = zone_xyzt[4 * (int64_t)z + 0], zy = zone_xyzt[4 * (int64_t)z + 1];
-    const double zzc = zone_xyzt[4 * (int64_t)z + 2], ztc = zone_xyzt[4 * (int64_t)z + 3];
-    const double zu = (lp.loctype == 1) ? zx : (lp.loctype == 2 ? zzc : ztc);
-    const double zv = (lp.loctype == 1) ? zy : 0.0;
-    const double L = corr_len[z], Rmax = max_len[z];
-    // the FP32 distance (relative error < 1e-6, sel::ZoneCell32) decides outside a 3e-6 band
-    const float r_lo = (float)Rmax * (1.f - 3e-6f), r_hi = (float)Rmax * (1.f + 3e-6f);
-    // the zone's FP64 set-up (divisions, floors) once, by one thread
-    if (tid == 0) {
-      ts.nrel = 0;
-      ts.bad = 0;
-      ts.zc = sel::zone_cell32(g, zu, zv, Rmax);
-      ts.iL = 1.0 / L;
-      if (full_scan) {
-        ts.sr.cu0 = 0;
-        ts.sr.cu1 = g.nu - 1;
-        ts.sr.cv0 = 0;
-        ts.sr.cv1 = g.nv - 1;
-        ts.sr.all_u = 1;
-      } else {
-        ts.sr = sel::zone_scan_range(g, lp.metric, lp.loctype, zu, zv, Rmax);
-      }
-    }
-    __syncthreads();  // ts.zc, ts.sr, ts.iL published (read only in this zone's scan)
-    const sel::ZoneCell32 zc = ts.zc;
-    const bool fastz = fast && zc.ok && !brute;  // brute force: one cell, no local offsets
-    const double iL = ts.iL, iL2 = iL * iL;
-    const float iL32 = (float)iL;
-    for (int e = tid; e < kLevelsExact * kTri; e += kThreads) acc64[e] = 0;
-    for (int e = tid; e < kTri; e += kThreads) accf[e] = 0.f;
-    int head = 0, tail = 0, ntile = 0, ctile = 0, nrel_local = 0, bad = 0;
-    double gsum = 0.0, gsum1 = 0.0;
-
-    // stage ring entries [head, head + rows) as one K-tile and issue its MMAs
-    auto do_tile = [&](int rows) {
-      if (ctile == kFlushTiles) {
-        if (pend0) drain(0);
-        if (pend1) drain(1);
-        __syncthreads();  // MMA completion and flag published
-        if (ts.flag) {
-          abort = true;
-          return;
-        }
-        flush();
-        ctile = 0;
-      }
-      const int b = ntile & 1;
-      if (b ? pend1 : pend0) drain(b);
-      __syncthreads();  // buffer free (flag published), ring entries visible
-      if (ts.flag) {
-        abort = true;
-        return;
-      }
-      unsigned char* tb = tiles + b * kBufBytes;
-#pragma unroll 1
-      for (int pass = 0; pass < KT / 8 / kStageGroups; pass++) {
-        const int chunk = kq + kStageGroups * pass;
-        uint32_t pk[kDigits][4];
-        // the chunk's 8 elements loaded first (independent loads in flight together)
-        double hv[8], sv[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int k = 8 * chunk + i;
-          hv[i] = 0.0;
-          sv[i] = 0.0;
-          if (k < rows && a < N) {
-            const int idx = (head + k) & (kRing - 1);
-            hv[i] = so.HSt[(int64_t)ts.ring_q[idx] * N + a];
-            sv[i] = ts.ring_s[idx];
-            // two accumulators (even / odd observations): shorter FMA chains
-            if (i & 1)
-              gsum1 = fma(hv[i], ts.ring_t[idx], gsum1);
-            else
-              gsum = fma(hv[i], ts.ring_t[idx], gsum);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-          unsigned long long U[2];
-#pragma unroll
-          for (int u = 0; u < 2; u++)
-            U[u] = (unsigned long long)fixed_prod(sv[i + u], hv[i + u], Ea, bad) + kDigitBias;
-          uint32_t d[kDigits];
-          digit_pairs(U[0], U[1], d);
-#pragma unroll
-          for (int p = 0; p < kDigits; p++) pk[p][i >> 1] = d[p];
-        }
-#pragma unroll
-        for (int p = 0; p < kDigits; p++)
-          *reinterpret_cast<uint4*>(tb + p * kSliceBytes + tile_off(a, chunk)) =
-              make_uint4(pk[p][0], pk[p][1], pk[p][2], pk[p][3]);
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();  // tile complete
-      if (tid == 0) {
+        phf[b] ^= 1u;
+        if (*(volatile int32_t*)&ts.stop) break;
+        const uint32_t acc0 = *(volatile int32_t*)&ts.first[b] ? 0u : 1u;
         fence_after();
-        const uint32_t base = tile_addr + b * kBufBytes;
+        const uint32_t B = tile_addr + b * kBufBytes;
 #pragma unroll 1
         for (int kk = 0; kk < KT / 16; kk++) {
-          const uint32_t ko = kk * 32;
-          const uint32_t acc0 = (ctile > 0 || kk > 0) ? 1u : 0u;
-          // levels 0..3, columns 64 L: A = [D_p ; D_p+1], B = D_0 .. D_(3-p) into L = p .. 3
-#pragma unroll
-          for (int p = 0; p < 4; p++)
-            mma_f16(tmem + 64 * p, make_desc(base + p * kSliceBytes + ko), make_desc(base + ko),
-                     idesc_f16(64u * (4 - p)), p == 0 ? acc0 : 1u);
-          // levels 4..6, columns 256 + 64 (L - 4): B = D_qlo .. D_qhi, q = L - p
-#pragma unroll
-          for (int p = 0; p < kDigits; p++) {
-            const int qlo = (4 - p > 0) ? 4 - p : 0;
-            const int qhi = (6 - p < kDigits - 1) ? 6 - p : kDigits - 1;
-            const int off = qlo - (4 - p);
-            mma_f16(tmem + 256 + 64 * off, make_desc(base + p * kSliceBytes + ko),
-                     make_desc(base + qlo * kSliceBytes + ko),
-                     idesc_f16(64u * (qhi - qlo + 1)), p == 0 ? acc0 : 1u);
+          const uint32_t ko = kk * 32, acc = kk > 0 ? 1u : acc0;
+          const uint64_t b0 = make_desc(B + ko), b4 = make_desc(B + 4 * kSliceBytes + ko);
+          mma_f16(tmem, b0, b0, idesc_f16(256), acc);        // p = 0, q = 0..3: blocks 0..3
+          mma_f16(tmem + 256, b0, b4, idesc_f16(192), acc);  // q = 4..6: blocks 4..6
+          uint64_t a = make_desc(B + 2 * kSliceBytes + ko);
+          mma_f16(tmem + 128, a, b0, idesc_f16(256), 1u);    // p = 2, q = 0..3: blocks 2..5
+          mma_f16(tmem + 384, a, b4, idesc_f16(64), 1u);     // q = 4: block 6
+          mma_f16(tmem + 448, a, make_desc(B + 5 * kSliceBytes + ko), idesc_f16(64), acc);
+          mma_f16(tmem + 256, b4, b0, idesc_f16(256), 1u);   // p = 4, q = 0..3: blocks 4..7
+          a = make_desc(B + 6 * kSliceBytes + ko);
+          mma_f16(tmem + 384, a, b0, idesc_f16(128), 1u);    // p = 6, q = 0, 1: blocks 6, 7
+        }
+        mma_commit(done0 + 8 * b);
+      }
+    }
+    __syncwarp();
+  } else if (warp == kThreads / 32 + 1) {
+    // ---- scout: picks the next zone and forms its FP64 set-up (divisions, floors: some 10,000
+    // cycles on one thread) while the workers are at the present one
+    for (int par = 0;; par ^= 1) {
+      int32_t w = 0;
+      if (lane == 0) {
+        OzZone& s = ts.zone[par];
+        w = atomicAdd(work, 1);  // pick number; zone order[z0 + w] when a pick order is given
+        s.w = w;
+        if (w < nzc) {
+          const int32_t zl = order ? order[z0 + w] : w;
+          const int32_t z = zlist ? zlist[w] : z0 + zl;  // a list's zones: slots in list order
+          s.zl = zl;
+          s.z = z;
+          const double zx = zone_xyzt[4 * (int64_t)z + 0], zy = zone_xyzt[4 * (int64_t)z + 1];
+          const double zzc = zone_xyzt[4 * (int64_t)z + 2], ztc = zone_xyzt[4 * (int64_t)z + 3];
+          s.zu = (lp.loctype == 1) ? zx : (lp.loctype == 2 ? zzc : ztc);
+          s.zv = (lp.loctype == 1) ? zy : 0.0;
+          s.L = corr_len[z];
+          s.Rmax = max_len[z];
+          s.zc = sel::zone_cell32(g, s.zu, s.zv, s.Rmax);
+          s.iL = 1.0 / s.L;
+          if (full_scan) {
+            s.sr.cu0 = 0;
+            s.sr.cu1 = g.nu - 1;
+            s.sr.cv0 = 0;
+            s.sr.cv1 = g.nv - 1;
+            s.sr.all_u = 1;
+          } else {
+            s.sr = sel::zone_scan_range(g, lp.metric, lp.loctype, s.zu, s.zv, s.Rmax);
           }
         }
-        mma_commit(mbar0 + 8 * b);
       }
-      if (b)
-        pend1 = 1;
-      else
-        pend0 = 1;
-      ntile++;
-      ctile++;
-      head += rows;
+      w = __shfl_sync(0xffffffffu, w, 0);
+      bar_zone();  // the zone handed over; the workers are past the one before the last
+      if (w >= nzc || *(volatile int32_t*)&ts.stop) break;
+    }
+  } else {
+    // ---- workers
+    const int a = tid & (NB - 1), kq = tid >> 6;  // staging: member a, 8-observation chunk kq
+    const int Ea = ts.E[a];
+    const bool fast = (lp.loctype != 1) || (lp.metric == OAKG_METRIC_CARTESIAN);
+    uint32_t phd[2] = {0u, 0u};      // parity of the buffer's next completion
+    bool pend[2] = {false, false};   // buffer handed over, its completion not yet waited for
+    uint32_t nt = 0;                 // K-tiles handed over so far (buffer nt & 1)
+    bool abort = false;
+
+    auto wait_done = [&](int b) {
+      if (pend[b]) {
+        if (!mbar_wait(done0 + 8 * b, phd[b])) late = true;
+        phd[b] ^= 1u;
+        pend[b] = false;
+      }
+    };
+    // Add the accumulators into the level sums (first: they start them; last: the zone's G goes to
+    // Gs instead). Level L's even-digit part is in lanes 0-63 of column block L, its odd part in
+    // lanes 64-127 of block L - 1. A part sums up to 4 products of at most 2^14 a row, so over 256
+    // rows every level is an exact integer (at most 2^24).
+    // Row j keeps columns c <= j; a thread of each half gives the partner half of its columns and
+    // keeps the other.
+    auto flush = [&](bool first, bool last, bool zbad) {
+      wait_done(0);
+      wait_done(1);
+      fence_after();
+      bar_workers();  // every warp has seen its completions: the buffers take the exchange
+      const int q = warp & 3, cg = warp >> 2;
+      const bool odd = q >= 2;
+      const int j = 32 * (q & 1) + lane, gi = 2 * cg + (odd ? 1 : 0), gg = 2 * cg + (odd ? 0 : 1);
+      const bool act = 16 * cg < 32 * ((q & 1) + 1);  // columns of the rows' lower triangle
+      const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+      // four levels' 8 columns: four loads, one wait
+      auto read4 = [&](uint32_t ta, uint32_t (&r)[32]) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+              : "=r"(r[8 * i]), "=r"(r[8 * i + 1]), "=r"(r[8 * i + 2]), "=r"(r[8 * i + 3]),
+                "=r"(r[8 * i + 4]), "=r"(r[8 * i + 5]), "=r"(r[8 * i + 6]), "=r"(r[8 * i + 7])
+              : "r"(ta + 64u * i));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int p = 0; p < 32; p += 16)
+          asm volatile(""
+                       : "+r"(r[p]), "+r"(r[p + 1]), "+r"(r[p + 2]), "+r"(r[p + 3]),
+                         "+r"(r[p + 4]), "+r"(r[p + 5]), "+r"(r[p + 6]), "+r"(r[p + 7]),
+                         "+r"(r[p + 8]), "+r"(r[p + 9]), "+r"(r[p + 10]), "+r"(r[p + 11]),
+                         "+r"(r[p + 12]), "+r"(r[p + 13]), "+r"(r[p + 14]), "+r"(r[p + 15])
+                       :
+                       : "memory");
+      };
+      auto read = [&](int c0, long long (&hi)[8], long long (&lo)[8]) {
+        uint32_t r[32];
+        // integers: below 2^22 the bits of x + 1.5 2^23 are 0x4B400000 + x (data); a conversion else
+        auto ints = [&]() {
+          float mx = 0.f;
+#pragma unroll
+          for (int i = 0; i < 32; i++) mx = fmaxf(mx, fabsf(__uint_as_float(r[i])));
+          if (__any_sync(0xffffffffu, !(mx < 4194304.f))) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) r[i] = (uint32_t)__float2int_rn(__uint_as_float(r[i]));
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+              r[i] = __float_as_uint(__uint_as_float(r[i]) + 12582912.f) - 0x4B400000u;
+          }
+        };
+        auto level = [&](int i) { return (long long)(int32_t)r[i]; };
+        // odd digits: levels 1..3 are in blocks 0..2 (level 0 has none), levels 4..7 in blocks 3..6
+        read4(tl + c0, r);
+        ints();
+#pragma unroll
+        for (int t = 0; t < 8; t++)
+          hi[t] = odd ? level(t) * 65536 + level(8 + t) * 256 + level(16 + t)
+                      : level(t) * 16777216 + level(8 + t) * 65536 + level(16 + t) * 256 + level(24 + t);
+        read4(tl + (odd ? 192u : 256u) + c0, r);
+        ints();
+#pragma unroll
+        for (int t = 0; t < 8; t++)  // in units of level 6
+          lo[t] = level(t) * 65536 + level(8 + t) * 256 + level(16 + t) + ((level(24 + t) + 128) >> 8);
+      };
+      long long hi[8], lo[8];
+      if (act) {
+        read(8 * gg, hi, lo);
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          xch[(8 * gg + t) * NB + j] = hi[t];
+          xcl[(8 * gg + t) * NB + j] = lo[t];
+        }
+        read(8 * gi, hi, lo);
+      }
+      fence_before();
+      bar_workers();  // exchanged; tensor memory read
+      if (act) {
+        const int tj = tri(j);
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const int c = 8 * gi + t;
+          if (c <= j) {
+            hi[t] += xch[c * NB + j];
+            lo[t] += xcl[c * NB + j];
+            if (!first) {
+              hi[t] += acc_hi[tj + c];
+              lo[t] += acc_lo[tj + c];
+            }
+            if (!last) {
+              acc_hi[tj + c] = hi[t];
+              acc_lo[tj + c] = lo[t];
+            }
+          }
+        }
+      }
+      bar_workers();  // the exchange is read: the buffers take G or tiles
+      if (last) {
+        if (act) {
+#pragma unroll
+          for (int t = 0; t < 8; t++) {
+            const int c = 8 * gi + t;
+            if (c <= j) {
+              // each sum is exact in FP64 (below 2^53 for up to 2^17 observations); the addition
+              // rounds
+              const int ex = ts.E[j] + ts.E[c];
+              double val = scaled_i64(hi[t], ex - 36) + scaled_i64(lo[t], ex - 60);
+              if (zbad) val = __longlong_as_double(0x7FF8000000000000ll);  // NaN: non-finite input
+              Gs[j * kLdG + c] = val;
+              Gs[c * kLdG + j] = val;
+            }
+          }
+        }
+        bar_workers();
+      }
     };
 
-    const sel::ScanRange sr = ts.sr;
-    // The zone's candidates are the observations of cell rows cv0..cv1, each row one or (a
-    // periodic u axis wrapping) two contiguous ranges of the cell-sorted order. Range ri is
-    // (row cv0 + ri / 2, part ri % 2); blocks of kThreads ranges are flattened into one index
-    // space (exclusive prefix of their lengths), so that a pass of kThreads threads takes
-    // kThreads candidates across rows in the order of the rows. The order, and so the ring
-    // and the selection, are those of a row-by-row scan.
-    const int nranges = 2 * (sr.cv1 - sr.cv0 + 1);
-    for (int rbase = 0; rbase < nranges && !abort; rbase += kThreads) {
-      {
-        const int ri = rbase + tid;
-        int32_t rq0 = 0, rlen = 0;
-        if (ri < nranges) {
-          const int cv = sr.cv0 + (ri >> 1), part = ri & 1;
-          int cu_a = 0, cu_b = -1;
-          if (sr.all_u) {
-            if (!part) cu_b = g.nu - 1;
-          } else if (!g.periodic_u) {
-            if (!part) {
-              cu_a = sr.cu0;
-              cu_b = sr.cu1;
-            }
-          } else {
-            const int a0 = sr.cu0, b0 = sr.cu1;
-            if (a0 < 0) {
-              cu_a = part ? 0 : a0 + g.nu;
-              cu_b = part ? b0 : g.nu - 1;
-            } else if (b0 >= g.nu) {
-              cu_a = part ? 0 : a0;
-              cu_b = part ? b0 - g.nu : g.nu - 1;
-            } else if (!part) {
-              cu_a = a0;
-              cu_b = b0;
-            }
-          }
-          const int64_t c_lo = (int64_t)cu_a + (int64_t)g.nu * cv;
-          const int64_t c_hi = (int64_t)cu_b + (int64_t)g.nu * cv;
-          if (c_lo <= c_hi && c_lo >= 0 && c_hi < ncells) {
-            rq0 = so.cell_start[c_lo];
-            rlen = so.cell_start[c_hi + 1] - rq0;
-          }
-        }
-        int incl = rlen;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += t;
-        }
-        if (lane == 31) ts.warp_cnt[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-          const int wsum = (lane < kThreads / 32) ? ts.warp_cnt[lane] : 0;
-          int winc = wsum;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, winc, o);
-            if (lane >= o) winc += t;
-          }
-          if (lane < kThreads / 32) ts.wpre[lane] = winc - wsum;
-          if (lane == 31) ts.rtotal = winc;
-        }
-        __syncthreads();
-        ts.rlo[tid] = rq0;
-        ts.roff[tid] = ts.wpre[warp] + incl - rlen;
-        __syncthreads();
+    for (int par = 0; !abort; par ^= 1) {
+      bar_zone();
+      const OzZone& zn = ts.zone[par];
+      if (zn.w >= nzc) break;
+      const int32_t zl = zn.zl, z = zn.z;
+      const double zu = zn.zu, zv = zn.zv, L = zn.L, Rmax = zn.Rmax;
+      // the FP32 distance (relative error < 1e-6, sel::ZoneCell32) decides outside a 3e-6 band
+      const float r_lo = (float)Rmax * (1.f - 3e-6f), r_hi = (float)Rmax * (1.f + 3e-6f);
+      const bool fastz = fast && zn.zc.ok && !brute;  // brute force: one cell, no local offsets
+      const double iL = zn.iL, iL2 = iL * iL;
+      const float iL32 = (float)iL;
+      if (tid == 0) {
+        ts.nrel = 0;
+        ts.bad = 0;
       }
-      const int32_t ncand = ts.rtotal;
-      const int nr = min(kThreads, nranges - rbase);
-      for (int32_t gb = 0; gb < ncand && !abort; gb += kThreads) {
-        const int32_t gi = gb + tid;
-        int32_t q = 0;
-        int cv = sr.cv0;
-        const bool valid = gi < ncand;
-        if (valid) {
-          // the last range starting at or before gi (empty ranges share the next one's start)
-          int lo_i = 0, hi_i = nr - 1;
-          while (lo_i < hi_i) {
-            const int mid = (lo_i + hi_i + 1) >> 1;
-            if (ts.roff[mid] <= gi) lo_i = mid;
-            else hi_i = mid - 1;
-          }
-          q = ts.rlo[lo_i] + (gi - ts.roff[lo_i]);
-          cv = sr.cv0 + ((rbase + lo_i) >> 1);
+      int head = 0, tail = 0, ntile = 0, ctile = 0, nflush = 0, nrel_local = 0, bad = 0;
+      double gsum = 0.0, gsum1 = 0.0;
+
+      // stage ring entries [head, head + rows) as one K-tile and hand it to the issuer
+      auto do_tile = [&](int rows) {
+        if (ctile == kFlushTiles) {
+          flush(nflush == 0, false, false);
+          nflush++;
+          ctile = 0;
         }
-        int sel = 0, rel = 0;
-        if (valid) {
-          // FP32 decisions away from the thresholds, the reference's FP64 evaluation near them
-          bool done = false;
-          if (fastz) {
-            const float d32 = sel::cell_distance32(zc, so, q, cv, lp.loctype == 1);
-            const int inside = (d32 <= r_lo) ? 1 : ((d32 >= r_hi) ? 0 : -1);
-            if (inside >= 0) {
-              const float r32 = d32 * iL32;
-              if (lp.weight == OAKG_WEIGHT_GAUSS_CUTOFF) {
-                rel = inside;
-                done = true;
-              } else if (r32 >= 2.f + 1e-5f) {  // locfun = 0
-                rel = 0;
-                done = true;
-              } else if (r32 <= 2.f - 1e-3f) {  // locfun > 3e-13, far above its FP64 rounding
-                rel = inside;
-                done = true;
+        const int b = (int)(nt & 1u);
+        wait_done(b);
+        unsigned char* tb = tiles + b * kBufBytes;
+        // the chunk's 8 elements loaded first (independent loads in flight together)
+        double hv[8];
+        const bool in = a < N;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int k = 8 * kq + i;
+          hv[i] = (k < rows && in)
+                      ? so.HSt[(int64_t)ts.ring_q[(head + k) & (kRing - 1)] * N + a] : 0.0;
+        }
+        long long F[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int idx = (head + 8 * kq + i) & (kRing - 1);
+          const bool ok = 8 * kq + i < rows;
+          F[i] = fixed_row(ok ? ts.ring_m[idx] : 0ull, ts.ring_e[idx], hv[i], Ea, bad);
+          // the innovation projection (two accumulators: shorter FMA chains)
+          const double tq = ok ? ts.ring_t[idx] : 0.0;
+          if (i & 1)
+            gsum1 = fma(hv[i], tq, gsum1);
+          else
+            gsum = fma(hv[i], tq, gsum);
+        }
+        stage_digits<kSliceBytes>(F, tb, tile_off(a, kq));
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        fence_before();
+        if (tid == 0) ts.first[b] = ctile == 0;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full0 + 8 * b);
+        pend[b] = true;
+        nt++;
+        ntile++;
+        ctile++;
+        head += rows;
+      };
+
+      const sel::ScanRange sr = zn.sr;
+      // The zone's candidates are the observations of cell rows cv0..cv1, each row one or (a
+      // periodic u axis wrapping) two contiguous ranges of the cell-sorted order. Range ri is
+      // (row cv0 + ri / 2, part ri % 2); blocks of kThreads ranges are flattened into one index
+      // space (exclusive prefix of their lengths), so that a pass of kThreads threads takes
+      // kThreads candidates across rows in the order of the rows. The order, and so the ring
+      // and the selection, are those of a row-by-row scan.
+      const int nranges = 2 * (sr.cv1 - sr.cv0 + 1);
+      for (int rbase = 0; rbase < nranges; rbase += kThreads) {
+        {
+          const int ri = rbase + tid;
+          int32_t rq0 = 0, rlen = 0;
+          if (ri < nranges) {
+            const int cv = sr.cv0 + (ri >> 1), part = ri & 1;
+            int cu_a = 0, cu_b = -1;
+            if (sr.all_u) {
+              if (!part) cu_b = g.nu - 1;
+            } else if (!g.periodic_u) {
+              if (!part) {
+                cu_a = sr.cu0;
+                cu_b = sr.cu1;
+              }
+            } else {
+              const int a0 = sr.cu0, b0 = sr.cu1;
+              if (a0 < 0) {
+                cu_a = part ? 0 : a0 + g.nu;
+                cu_b = part ? b0 : g.nu - 1;
+              } else if (b0 >= g.nu) {
+                cu_a = part ? 0 : a0;
+                cu_b = part ? b0 - g.nu : g.nu - 1;
+              } else if (!part) {
+                cu_a = a0;
+                cu_b = b0;
               }
             }
+            const int64_t c_lo = (int64_t)cu_a + (int64_t)g.nu * cv;
+            const int64_t c_hi = (int64_t)cu_b + (int64_t)g.nu * cv;
+            if (c_lo <= c_hi && c_lo >= 0 && c_hi < ncells) {
+              rq0 = so.cell_start[c_lo];
+              rlen = so.cell_start[c_hi + 1] - rq0;
+            }
           }
-          if (!done) {
-            double d;
-            if (lp.loctype == 1)
-              d = sel::distance(so.u[q], so.v[q], zu, zv, lp.metric);
-            else
-              d = fabs(__dsub_rn(so.u[q], zu));
-            if (lp.weight == OAKG_WEIGHT_GAUSS_CUTOFF) {
-              rel = (d <= Rmax);
+          int incl = rlen;
+  #pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          if (lane == 31) ts.warp_cnt[warp] = incl;
+          bar_workers();
+          if (warp == 0) {
+            const int wsum = (lane < kThreads / 32) ? ts.warp_cnt[lane] : 0;
+            int winc = wsum;
+  #pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const int t = __shfl_up_sync(0xffffffffu, winc, o);
+              if (lane >= o) winc += t;
+            }
+            if (lane < kThreads / 32) ts.wpre[lane] = winc - wsum;
+            if (lane == 31) ts.rtotal = winc;
+          }
+          bar_workers();
+          ts.rlo[tid] = rq0;
+          ts.roff[tid] = ts.wpre[warp] + incl - rlen;
+          bar_workers();
+        }
+        const int32_t ncand = ts.rtotal;
+        const int nr = min(kThreads, nranges - rbase);
+        for (int32_t gb = 0; gb < ncand; gb += kThreads) {
+          const int32_t gi = gb + tid;
+          int32_t q = 0;
+          int cv = sr.cv0;
+          const bool valid = gi < ncand;
+          if (valid) {
+            // the last range starting at or before gi (empty ranges share the next one's start)
+            int lo_i = 0, hi_i = nr - 1;
+            while (lo_i < hi_i) {
+              const int mid = (lo_i + hi_i + 1) >> 1;
+              if (ts.roff[mid] <= gi) lo_i = mid;
+              else hi_i = mid - 1;
+            }
+            q = ts.rlo[lo_i] + (gi - ts.roff[lo_i]);
+            cv = sr.cv0 + ((rbase + lo_i) >> 1);
+          }
+          int sel = 0, rel = 0;
+          if (valid) {
+            // FP32 decisions away from the thresholds, the reference's FP64 evaluation near them
+            bool done = false;
+            if (fastz) {
+              const float d32 = sel::cell_distance32(zn.zc, so, q, cv, lp.loctype == 1);
+              const int inside = (d32 <= r_lo) ? 1 : ((d32 >= r_hi) ? 0 : -1);
+              if (inside >= 0) {
+                const float r32 = d32 * iL32;
+                if (lp.weight == OAKG_WEIGHT_GAUSS_CUTOFF) {
+                  rel = inside;
+                  done = true;
+                } else if (r32 >= 2.f + 1e-5f) {  // locfun = 0
+                  rel = 0;
+                  done = true;
+                } else if (r32 <= 2.f - 1e-3f) {  // locfun > 3e-13, far above its FP64 rounding
+                  rel = inside;
+                  done = true;
+                }
+              }
+            }
+            if (!done) {
+              double d;
+              if (lp.loctype == 1)
+                d = sel::distance(so.u[q], so.v[q], zu, zv, lp.metric);
+              else
+                d = fabs(__dsub_rn(so.u[q], zu));
+              if (lp.weight == OAKG_WEIGHT_GAUSS_CUTOFF) {
+                rel = (d <= Rmax);
+              } else {
+                rel = (d <= Rmax) && (sel::locfun(d / L) != 0.0);
+              }
+            }
+            sel = rel || !lp.localise;
+          }
+          nrel_local += rel;
+          const unsigned ball = __ballot_sync(0xffffffffu, sel);
+          if (lane == 0) ts.warp_cnt[warp] = __popc(ball);
+          bar_workers();
+          int before = 0, total = 0;
+  #pragma unroll
+          for (int w2 = 0; w2 < kThreads / 32; w2++) {
+            const int cnt = ts.warp_cnt[w2];
+            before += (w2 < warp) ? cnt : 0;
+            total += cnt;
+          }
+          if (sel) {
+            const int slot = (tail + before + __popc(ball & ((1u << lane) - 1u))) & (kRing - 1);
+            ts.ring_q[slot] = q;
+          }
+          bar_workers();
+          // the plain form's FP64 weights of the new entries (zone_gram.cu), one thread an
+          // entry, so that the FP64 work runs with full warps: sqrt(c) = |w| / sqrt(r)
+          // (c = w (w / r), DCDCovar, covariance.F90:612-619) and c (yo - Hxf). The values
+          // (not the decisions, made above with the reference's rounding) are evaluated with
+          // fewer FP64 operations for the Cartesian and 1-D distances: exp(-d^2 / L^2) needs
+          // no square root or division, locfun(sqrt(d^2) / L) takes 1/L once a zone.
+          if (tid < total) {
+            const int slot = (tail + tid) & (kRing - 1);
+            const int32_t qs = ts.ring_q[slot];
+            double w64;
+            if (fast) {
+              const double du = so.u[qs] - zu;
+              double D2 = du * du;
+              if (lp.loctype == 1) {
+                const double dv = so.v[qs] - zv;
+                D2 = fma(dv, dv, D2);
+              }
+              w64 = (lp.weight == OAKG_WEIGHT_GAUSS_CUTOFF) ? exp(-(D2 * iL2))
+                                                            : sel::locfun_value(sqrt(D2) * iL);
             } else {
-              rel = (d <= Rmax) && (sel::locfun(d / L) != 0.0);
+              double d;
+              if (lp.loctype == 1)
+                d = sel::distance(so.u[qs], so.v[qs], zu, zv, lp.metric);
+              else
+                d = fabs(__dsub_rn(so.u[qs], zu));
+              if (lp.weight == OAKG_WEIGHT_GAUSS_CUTOFF) {
+                const double t = d / L;
+                w64 = exp(-(t * t));
+              } else {
+                w64 = sel::locfun(d / L);
+              }
             }
+            const double sc = fabs(w64) * isr[qs];
+            const unsigned long long sb = (unsigned long long)__double_as_longlong(sc);
+            const int es = (int)(sb >> 52) & 0x7FF;
+            ts.ring_m[slot] = es ? ((sb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11 : 0ull;
+            ts.ring_e[slot] = es;
+            if (es == 0x7FF) bad = 1;  // (sc >= 0: no sign)
+            ts.ring_t[slot] = sc * sc * so.innov[qs];
           }
-          sel = rel || !lp.localise;
+          tail += total;
+          bar_workers();  // the new entries and their weights are visible
+          while (tail - head >= KT) do_tile(KT);
         }
-        nrel_local += rel;
-        const unsigned ball = __ballot_sync(0xffffffffu, sel);
-        if (lane == 0) ts.warp_cnt[warp] = __popc(ball);
-        __syncthreads();
-        int before = 0, total = 0;
+        bar_workers();  // the block's ranges consumed before the next block overwrites them
+      }
+      if (tail > head) do_tile(tail - head);
+      // relevant-observation count of the zone
+      for (int o = 16; o > 0; o >>= 1) nrel_local += __shfl_xor_sync(0xffffffffu, nrel_local, o);
+      if (lane == 0) atomicAdd(&ts.nrel, nrel_local);
+      if (bad) atomicOr(&ts.bad, 1);
+      gpart[kq * NB + a] = gsum + gsum1;
+      bar_workers();  // nrel, bad and the partials published
+      const int nrel = ts.nrel;
+      if (tid == 0) nobs[z] = nrel;
+      if (ctile > 0) flush(nflush == 0, true, ts.bad != 0);
+      if (nrel > 0 && ntile > 0) {
+        double* Gz = G + (int64_t)zl * N * N;
+        for (int idx = tid; idx < N * NB; idx += kThreads) {
+          const int j = idx >> 6, c = idx & (NB - 1);
+          if (c < N) Gz[j * N + c] = Gs[j * kLdG + c];
+        }
+        if (tid < N) {
+          double gs = 0.0;
 #pragma unroll
-        for (int w2 = 0; w2 < kThreads / 32; w2++) {
-          const int cnt = ts.warp_cnt[w2];
-          before += (w2 < warp) ? cnt : 0;
-          total += cnt;
+          for (int p = 0; p < kStageGroups; p++) gs += gpart[p * NB + tid];
+          gv[(int64_t)zl * N + tid] = gs;
         }
-        if (sel) {
-          const int slot = (tail + before + __popc(ball & ((1u << lane) - 1u))) & (kRing - 1);
-          ts.ring_q[slot] = q;
-        }
-        __syncthreads();
-        // the plain form's FP64 weights of the new entries (zone_gram.cu), one thread an
-        // entry, so that the FP64 work runs with full warps: sqrt(c) = |w| / sqrt(r)
-        // (c = w (w / r), DCDCovar, covariance.F90:612-619) and c (yo - Hxf). The values
-        // (not the decisions, made above with the reference's rounding) are evaluated with
-        // fewer FP64 operations for the Cartesian and 1-D distances: exp(-d^2 / L^2) needs
-        // no square root or division, locfun(sqrt(d^2) / L) takes 1/L once a zone.
-        if (tid < total) {
-          const int slot = (tail + tid) & (kRing - 1);
-          const int32_t qs = ts.ring_q[slot];
-          double w64;
-          if (fast) {
-            const double du = so.u[qs] - zu;
-            double D2 = du * du;
-            if (lp.loctype == 1) {
-              const double dv = so.v[qs] - zv;
-              D2 = fma(dv, dv, D2);
-            }
-            w64 = (lp.weight == OAKG_WEIGHT_GAUSS_CUTOFF) ? exp(-(D2 * iL2))
-                                                          : sel::locfun_value(sqrt(D2) * iL);
-          } else {
-            double d;
-            if (lp.loctype == 1)
-              d = sel::distance(so.u[qs], so.v[qs], zu, zv, lp.metric);
-            else
-              d = fabs(__dsub_rn(so.u[qs], zu));
-            if (lp.weight == OAKG_WEIGHT_GAUSS_CUTOFF) {
-              const double t = d / L;
-              w64 = exp(-(t * t));
-            } else {
-              w64 = sel::locfun(d / L);
-            }
-          }
-          const double sc = fabs(w64) * isr[qs];
-          ts.ring_s[slot] = sc;
-          ts.ring_t[slot] = sc * sc * so.innov[qs];
-        }
-        tail += total;
-        while (tail - head >= KT && !abort) do_tile(KT);
       }
-      __syncthreads();  // the block's ranges consumed before the next block overwrites them
+      // uniform: a wait that expired in any thread ends the workers
+      int any;
+      asm volatile(
+          "{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\n"
+          "selp.s32 %0, 1, 0, q;\n}\n"
+          : "=r"(any)
+          : "r"((int)late), "n"(kThreads)
+          : "memory");
+      abort = any != 0;
     }
-    if (!abort && tail > head) do_tile(tail - head);
-    if (abort) break;
-    // relevant-observation count of the zone
-    for (int o = 16; o > 0; o >>= 1) nrel_local += __shfl_xor_sync(0xffffffffu, nrel_local, o);
-    if (lane == 0) atomicAdd(&ts.nrel, nrel_local);
-    if (bad) atomicOr(&ts.bad, 1);
-    gpart[kq * NB + a] = gsum + gsum1;
-    if (ntile > 0) {
-      if (pend0) drain(0);
-      if (pend1) drain(1);
-    }
-    __syncthreads();  // nrel, bad, partials and the MMA completion published
-    if (ts.flag) break;
-    const int nrel = ts.nrel;
-    if (tid == 0) nobs[z] = nrel;
-    if (nrel > 0 && ntile > 0) {
-      flush();
-      double* Gz = G + (int64_t)zl * N * N;
-      const bool zbad = ts.bad != 0;
-      for (int e = tid; e < kTri; e += kThreads) {
-        int j = (int)((__fsqrt_rn((float)(8 * e + 1)) - 1.0f) * 0.5f);
-        while ((j + 1) * (j + 2) / 2 <= e) j++;
-        while (j * (j + 1) / 2 > e) j--;
-        const int c = e - tri(j);
-        if (j >= N) continue;
-        const long long v =
-            ((acc64[e] * 256 + acc64[kTri + e]) * 256 + acc64[2 * kTri + e]) * 256 +
-            acc64[3 * kTri + e];
-        // 2^(E_j + E_c - 36), a power of two in the normal range for any practical scale
-        int ex = ts.E[j] + ts.E[c] - 36 + 1023;
-        ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
-        const double scale = __longlong_as_double((long long)ex << 52);
-        double val = fma((double)accf[e], 1.0 / 256.0, (double)v) * scale;
-        if (zbad) val = __longlong_as_double(0x7FF8000000000000ll);  // NaN: non-finite input
-        Gz[j * N + c] = val;
-        Gz[c * N + j] = val;
-      }
-      if (tid < N) {
-        double gs = 0.0;
-#pragma unroll
-        for (int p = 0; p < kStageGroups; p++) gs += gpart[p * NB + tid];
-        gv[(int64_t)zl * N + tid] = gs;
-      }
-    }
-    __syncthreads();  // G staging and partials consumed before the next zone's tiles
+    // release the issuer, and after an expired wait the scout
+    if (tid == 0) ts.stop = 1;
+    __syncwarp();
+    bar_workers();
+    if (lane == 0) mbar_arrive(full0 + 8 * (nt & 1u));
+    if (abort) bar_zone();
+    wait_done(0);
+    wait_done(1);
   }
   // teardown: no MMA may still write tensor memory when it is freed
-  if (pend0) drain(0);
-  if (pend1) drain(1);
-  if (tid == 0 && ts.flag) atomicOr(err, ZST_TIMEOUT);
+  if (late) atomicOr(err, ZST_TIMEOUT);
   fence_before();
   __syncthreads();
   fence_after();
@@ -697,7 +822,7 @@ __global__ void k_oz_exponents(int N, const unsigned long long* __restrict__ mx,
 // the rotation's sums and update). The shared-memory request keeps a second CTA (which would
 // wait for the tensor memory) off the SM.
 constexpr int kTsLd = NB + 1;
-constexpr size_t kTsData = 1024 + (size_t)kBufBytes + kSliceBytes +
+constexpr size_t kTsData = 1024 + (size_t)kBufBytes +
                            (size_t)NB * kTsLd * sizeof(double) + (size_t)NB * NB * sizeof(double) +
                            18 * NB * sizeof(double);
 constexpr size_t kTsDynSmem = (size_t)148 * 1024;
@@ -754,7 +879,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t pad = ((raw_addr + 1023u) & ~1023u) - raw_addr;
   unsigned char* tile = dyn_raw + pad;  // the 7 slices and the zero slice past them
   const uint32_t tile_addr = raw_addr + pad;
-  double* Ts = reinterpret_cast<double*>(tile + kBufBytes + kSliceBytes);  // [NB][kTsLd]
+  double* Ts = reinterpret_cast<double*>(tile + kBufBytes);  // [NB][kTsLd]
   double* Upre = Ts + NB * kTsLd;  // next zone's U slot, as stored (U_ak at k N + a)
   double* qpre = Upre + NB * NB;   // next zone's (1 + lambda)^-1/4
   double* vpre = qpre + NB;        // next zone's v
@@ -776,7 +901,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (tid < NB) ts.emax[tid] = 0;
   // rows 64-127 of the last digit's A operand: read by the MMA, never read back
   for (uint32_t i = tid; i < kSliceBytes / 16; i += kThreads)
-    reinterpret_cast<uint4*>(tile + kBufBytes)[i] = make_uint4(0, 0, 0, 0);
+    reinterpret_cast<uint4*>(tile + 7 * kSliceBytes)[i] = make_uint4(0, 0, 0, 0);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&ts.tmem_base)),
@@ -1003,7 +1128,7 @@ cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int 
                          int32_t z0, int32_t nzc, const double* zone_xyzt, const double* corr_len,
                          const double* max_len, double* d_G, double* d_g, int32_t* d_nobs,
                          int brute, int32_t* d_work, int32_t* d_err, void* d_scratch,
-                         cudaStream_t st, const int32_t* order) {
+                         cudaStream_t st, const int32_t* order, const int32_t* zlist) {
   if (N < 1 || N > NB || !so.HSt || !so.r || !d_scratch) return cudaErrorInvalidValue;
   unsigned long long* mx = reinterpret_cast<unsigned long long*>(d_scratch);
   int32_t* E = reinterpret_cast<int32_t*>(mx + NB);
@@ -1033,9 +1158,9 @@ cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int 
   if (grid > nzc) grid = nzc > 0 ? nzc : 1;
   e = cudaMemsetAsync(d_work, 0, sizeof(int32_t), st);
   if (e != cudaSuccess) return e;
-  k_zone_gram_oz<<<grid, kThreads, kDynSmem, st>>>(g, so, N, lp, z0, nzc, zone_xyzt, corr_len,
+  k_zone_gram_oz<<<grid, kThreads + 64, kDynSmem, st>>>(g, so, N, lp, z0, nzc, zone_xyzt, corr_len,
                                                    max_len, E, isr, d_G, d_g, d_nobs, brute,
-                                                   d_work, d_err, order);
+                                                   d_work, d_err, order, zlist);
   count_launches(1);
   return cudaGetLastError();
 }
