@@ -989,11 +989,21 @@ int adjoint_impl(const oakg_dims* dims, const oakg_loc* loc, int32_t Z, const in
     if ((rc = scratch(c, B_G, (size_t)chunk * N * N, &d_G, "zone matrices"))) return rc;
     if ((rc = scratch(c, B_GV, (size_t)chunk * N, &d_gv, "zone vectors"))) return rc;
   }
+  unsigned char* d_oz = nullptr;
+  if (N <= gram_oz_max_n() && m > 0 && !(lp.flags & OAKG_FLAG_SIMT_GRAM) &&
+      (rc = scratch(c, B_OZSCR, gram_oz_scratch_bytes(m), &d_oz, "Gram exponents")))
+    return rc;
+  cudaMemsetAsync(d_work + 2, 0, sizeof(int32_t), st);  // device status of the Gram
   cudaEventRecord(c->ev[1], st);
   for (int64_t k0 = 0; k0 < nact; k0 += chunk) {
     const int32_t nk = (int32_t)std::min<int64_t>(chunk, nact - k0);
-    e = zone_gram_fp64_list(P.g, P.so, N, lp, d_list + k0, nk, P.zxyzt, P.corr, P.maxl, d_G, d_gv,
-                            d_nobs, P.brute, d_work, st);
+    // the forward's Gram (ZoneKernels<double>::gram) on the list
+    if (d_oz)
+      e = zone_gram_oz(P.g, P.so, m, N, lp, 0, nk, P.zxyzt, P.corr, P.maxl, d_G, d_gv, d_nobs,
+                       P.brute, d_work, d_work + 2, d_oz, st, nullptr, d_list + k0);
+    else
+      e = zone_gram_fp64_list(P.g, P.so, N, lp, d_list + k0, nk, P.zxyzt, P.corr, P.maxl, d_G,
+                              d_gv, d_nobs, P.brute, d_work, st);
     if (e != cudaSuccess) return cuda_fail(e, "selection/Gram kernel");
     e = zone_adjoint_fp64(P.g, P.so, N, lp, d_list + k0, nk, P.zxyzt, P.corr, P.maxl, P.zstart,
                           P.Sf, ldS, d_seed, inflation, d_G, d_gv, d_nobs, d_dyo, d_dr, d_scal,
@@ -1004,6 +1014,9 @@ int adjoint_impl(const oakg_dims* dims, const oakg_loc* loc, int32_t Z, const in
   double hs[2] = {0, 0};
   if ((e = cudaMemcpyAsync(hs, d_scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, st)))
     return cuda_fail(e, "D2H");
+  int32_t hstatus = 0;
+  if ((e = cudaMemcpyAsync(&hstatus, d_work + 2, sizeof(int32_t), cudaMemcpyDeviceToHost, st)))
+    return cuda_fail(e, "D2H");
   if (mem == OAKG_MEM_HOST && m > 0) {
     if (dJ_dyo && (e = cudaMemcpyAsync(dJ_dyo, d_dyo, m * sizeof(double), cudaMemcpyDeviceToHost,
                                        st)))
@@ -1013,6 +1026,7 @@ int adjoint_impl(const oakg_dims* dims, const oakg_loc* loc, int32_t Z, const in
       return cuda_fail(e, "D2H dJ_dr");
   }
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "synchronize");
+  if ((rc = status_code(hstatus))) return rc;
   if (dJ_dlen) *dJ_dlen = hs[0];
   if (dJ_dinfl) *dJ_dinfl = hs[1];
   c->timings[0] = elapsed(c->ev[0], c->ev[1]);

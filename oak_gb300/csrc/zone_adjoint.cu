@@ -17,7 +17,12 @@
 // weight and its slope vanish at the cut-off, so nothing is lost there.
 //
 // A is factorised per zone (Cholesky, in shared memory) from G recomputed by the forward
-// selection + Gram kernel for the seeded zones only; no eigensystem is stored.
+// selection + Gram kernel for the seeded zones only (up to 64 members the tensor-core kernel on
+// the list, as in the forward; the FP64 list kernel above that, and where it is asked for); no
+// eigensystem is stored. The factorisation was a chain of divisions, square roots and block
+// barriers: the right-hand sides now ride along as two extra rows (no forward substitution), the
+// pivot's reciprocal root is one thread's, and the back substitution goes by columns. 2,400
+// seeded zones of 64,800, N = 64, the whole call: 7.5 to 8.2 ms before, 3.3 ms now.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -62,35 +67,11 @@ __global__ void k_zone_flags(const double* __restrict__ seed,
   }
 }
 
-// one block: exclusive scan of the flags -> positions, then the compacted zone list;
-// pos[Z] = number of seeded zones
-__global__ void k_zone_compact(const int32_t* __restrict__ flag, int32_t Z,
-                               int32_t* __restrict__ pos, int32_t* __restrict__ list) {
-  __shared__ int32_t s[1024];
-  __shared__ int32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int32_t base = 0; base < Z; base += 1024) {
-    const int32_t i = base + threadIdx.x;
-    const int32_t x = (i < Z) ? flag[i] : 0;
-    s[threadIdx.x] = x;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-      int32_t t = (threadIdx.x >= off) ? s[threadIdx.x - off] : 0;
-      __syncthreads();
-      s[threadIdx.x] += t;
-      __syncthreads();
-    }
-    const int32_t p = carry + s[threadIdx.x] - x;
-    if (i < Z) {
-      pos[i] = p;
-      if (x) list[p] = i;
-    }
-    __syncthreads();
-    if (threadIdx.x == 1023) carry += s[1023];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) pos[Z] = carry;
+// the seeded zones in order, from the exclusive scan of their flags
+__global__ void k_zone_list(const int32_t* __restrict__ flag, const int32_t* __restrict__ pos,
+                            int32_t Z, int32_t* __restrict__ list) {
+  for (int32_t z = blockIdx.x * blockDim.x + threadIdx.x; z < Z; z += gridDim.x * blockDim.x)
+    if (flag[z]) list[pos[z]] = z;
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -105,9 +86,11 @@ __global__ void __launch_bounds__(kThreads)
                    int32_t* __restrict__ work) {
   extern __shared__ double dyn[];
   const int ld = N + 1;
-  double* A = dyn;           // [N][ld] I + s^2 G, then its Cholesky factor L (lower)
-  double* am = A + N * ld;   // [N] ampl = A^-1 s g
-  double* y = am + N;        // [N] A^-1 b
+  double* A = dyn;                 // [N + 2][ld] I + s^2 G, then its Cholesky factor L (lower);
+                                   // rows N and N + 1: the right-hand sides s g and b
+  double* am = A + (N + 2) * ld;   // [N] ampl = A^-1 s g
+  double* y = am + N;              // [N] A^-1 b
+  double* invd = y + N;            // [N] 1 / L_kk
   __shared__ double red[kWarps + 1];
   __shared__ int32_t s_zone;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -129,57 +112,58 @@ __global__ void __launch_bounds__(kThreads)
       A[i * ld + j] = s * s * Gz[idx] + ((i == j) ? 1.0 : 0.0);
     }
     const int64_t i1 = zone_start[z], i2 = zone_start[z + 1];
-    // am <- s g, y <- b = s Sf_z^T a
-    for (int k = tid; k < N; k += kThreads) {
-      am[k] = s * gv[(int64_t)zl * N + k];
+    // rows N: s g, N + 1: b = s Sf_z^T a (N <= kThreads: one member a thread)
+    double bk = 0.0;
+    if (tid < N) {
+      A[N * ld + tid] = s * gv[(int64_t)zl * N + tid];
       double acc = 0.0;
-      for (int64_t i = i1; i < i2; i++) acc = fma(Sf[i + (int64_t)k * ldS], seed[i], acc);
-      y[k] = s * acc;
+      for (int64_t i = i1; i < i2; i++) acc = fma(Sf[i + (int64_t)tid * ldS], seed[i], acc);
+      bk = s * acc;
+      A[(N + 1) * ld + tid] = bk;
     }
     __syncthreads();
-    // Cholesky A = L L^T (right-looking, lower triangle)
+    // Cholesky A = L L^T (right-looking, lower triangle) with the two right-hand sides as further
+    // rows, which it turns into L^-1 s g and L^-1 b. The reciprocal root of a pivot is formed by
+    // one warp for all (by every warp it is the FP64 pipe's largest item).
     for (int k = 0; k < N; k++) {
-      if (tid == 0) A[k * ld + k] = sqrt(A[k * ld + k]);
+      if (tid == 0) invd[k] = rsqrt(A[k * ld + k]);
       __syncthreads();
-      const double inv = 1.0 / A[k * ld + k];
-      for (int i = k + 1 + tid; i < N; i += kThreads) A[i * ld + k] *= inv;
+      const double inv = invd[k];
+      for (int i = k + 1 + tid; i < N + 2; i += kThreads) A[i * ld + k] *= inv;
       __syncthreads();
-      const int L = N - k - 1;
-      for (int idx = tid; idx < L * L; idx += kThreads) {
-        int i = idx / L, j = idx - i * L;
-        if (j <= i) {
-          double* a = A + (k + 1 + i) * ld + (k + 1 + j);
-          *a = fma(-A[(k + 1 + i) * ld + k], A[(k + 1 + j) * ld + k], *a);
+      // rows k + 1 .. N + 1, columns k + 1 .. min(row, N - 1)
+      const int L = N - k - 1, E = L * (L + 1) / 2;
+      for (int e2 = tid; e2 < E + 2 * L; e2 += kThreads) {
+        int i, j;
+        if (e2 < E) {
+          i = (int)((__fsqrt_rn((float)(8 * e2 + 1)) - 1.0f) * 0.5f);
+          while ((i + 1) * (i + 2) / 2 <= e2) i++;
+          while (i * (i + 1) / 2 > e2) i--;
+          j = e2 - i * (i + 1) / 2;
+        } else {
+          const int r = e2 - E;
+          i = r < L ? L : L + 1;
+          j = r < L ? r : r - L;
         }
+        double* a = A + (k + 1 + i) * ld + (k + 1 + j);
+        *a = fma(-A[(k + 1 + i) * ld + k], A[(k + 1 + j) * ld + k], *a);
       }
       __syncthreads();
     }
-    // two right-hand sides: L L^T am = s g, L L^T y = b (warp 0 per system, lanes over k)
+    // L^T x = z for both, one warp each, by columns (no reduction on the way)
     if (warp < 2) {
       double* x = (warp == 0) ? am : y;
-      for (int i = 0; i < N; i++) {  // forward: L z = rhs
-        double t = 0.0;
-        for (int k = lane; k < i; k += 32) t = fma(A[i * ld + k], x[k], t);
-        t = warp_sum(t);
-        if (lane == 0) x[i] = (x[i] - t) / A[i * ld + i];
-        __syncwarp();
-      }
-      for (int i = N - 1; i >= 0; i--) {  // backward: L^T x = z
-        double t = 0.0;
-        for (int k = i + 1 + lane; k < N; k += 32) t = fma(A[k * ld + i], x[k], t);
-        t = warp_sum(t);
-        if (lane == 0) x[i] = (x[i] - t) / A[i * ld + i];
+      double* zr = A + (N + warp) * ld;
+      for (int i = N - 1; i >= 0; i--) {
+        const double xi = zr[i] * invd[i];
+        if (lane == 0) x[i] = xi;
+        for (int k = lane; k < i; k += 32) zr[k] = fma(-A[i * ld + k], xi, zr[k]);
         __syncwarp();
       }
     }
     __syncthreads();
-    // b^T ampl = s a^T Sf ampl (the direct part of dJ/ds): recompute b per k
-    double part = 0.0;
-    for (int k = tid; k < N; k += kThreads) {
-      double acc = 0.0;
-      for (int64_t i = i1; i < i2; i++) acc = fma(Sf[i + (int64_t)k * ldS], seed[i], acc);
-      part = fma(s * acc, am[k], part);
-    }
+    // b^T ampl = s a^T Sf ampl (the direct part of dJ/ds)
+    double part = (tid < N) ? bk * am[tid] : 0.0;
     // re-run the zone's selection; every relevant observation adds its terms
     const double zx = zone_xyzt[4 * (int64_t)z + 0], zy = zone_xyzt[4 * (int64_t)z + 1];
     const double zzc = zone_xyzt[4 * (int64_t)z + 2], ztc = zone_xyzt[4 * (int64_t)z + 3];
@@ -281,7 +265,9 @@ cudaError_t zone_active_list(const double* seed, const int64_t* zone_start, int3
   if (grid > 152 * 8) grid = 152 * 8;
   if (grid < 1) grid = 1;
   k_zone_flags<<<grid, 256, 0, st>>>(seed, zone_start, Z, d_flag);
-  k_zone_compact<<<1, 1024, 0, st>>>(d_flag, Z, d_pos, d_list);
+  const cudaError_t e = scan_exclusive_i32(d_flag, Z, d_pos, st);
+  if (e != cudaSuccess) return e;
+  k_zone_list<<<grid, 256, 0, st>>>(d_flag, d_pos, Z, d_list);
   count_launches(2);
   return cudaGetLastError();
 }
@@ -293,7 +279,7 @@ cudaError_t zone_adjoint_fp64(const CellGrid& g, const SortedObs& so, int N, Loc
                               const double* seed, double infl, const double* d_G,
                               const double* d_g, const int32_t* d_nobs, double* dyo, double* dr,
                               double* dscal, int brute, int32_t* d_work, cudaStream_t st) {
-  size_t smem = (size_t)(N * (N + 1) + 2 * N) * sizeof(double);
+  size_t smem = (size_t)((N + 2) * (N + 1) + 3 * N) * sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(k_zone_adjoint,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
