@@ -208,6 +208,14 @@ int isqrt_oz_max_n();
 cudaError_t zone_isqrt_oz(int N, int32_t nzc, double* d_GT, const float* d_V, const float* d_aux32,
                           const double* d_g, const int32_t* d_nobs, int rotate, double* d_ampl,
                           int32_t* d_status, int32_t* d_retries, cudaStream_t st);
+// ---- zone_sqrt64.cu: the same from the tridiagonal form and the reflectors that E1 of the FP64
+// eigensolve left in d_aux (aux_stride doubles a zone) and in G's strict lower triangle, for
+// 3 <= N <= sqrt64_max_n(). ZST_RETRY (counted in *d_retries) where it leaves a zone to the
+// eigenvalue stages, with both as they were; *d_work: a zero counter.
+int sqrt64_max_n();
+cudaError_t zone_sqrt64(int N, int32_t nzc, double* d_GT, const double* d_aux, int aux_stride,
+                        const double* d_g, const int32_t* d_nobs, int rotate, double* d_ampl,
+                        int32_t* d_status, int32_t* d_work, int32_t* d_retries, cudaStream_t st);
 // zone_eig_fp32 with the FP32 eigenpairs refined to FP64 accuracy (Ogita-Aishima) before T and
 // the amplitudes are formed (zone_refine.cu): d_G0 (N x N floats a zone) keeps G, d_S holds
 // zone_refine_scratch(N) floats a zone; N <= 128.

@@ -88,6 +88,24 @@ __device__ __forceinline__ R warp_sum(R x) {
   return x;
 }
 
+// sqrt(x) and 2 / x: FP64 inside FP32's range from the FP32 value by the series of
+// (1 - e)^(-1/2) and 1 / (1 - e) to the second order (e below 2^-20: five and three FP64
+// operations on the chain of every reflector)
+__device__ __forceinline__ float sqrt_of(float x) { return sqrtf(x); }
+__device__ __forceinline__ double sqrt_of(double x) {
+  const float f = (float)x;
+  if (!(f > 1e-30f && f < 1e30f)) return sqrt(x);
+  const double r = (double)rsqrtf(f), t = x * r, e = fma(-t, r, 1.0);
+  return fma(t * e, fma(e, 0.375, 0.5), t);
+}
+__device__ __forceinline__ float two_over(float x) { return 2.f / x; }
+__device__ __forceinline__ double two_over(double x) {
+  const float f = (float)x;
+  if (!(f > 1e-30f && f < 1e30f)) return 2.0 / x;
+  const double r = (double)__fdividef(1.f, f), e = fma(-x, r, 1.0), t = 2.0 * r;
+  return fma(t, fma(e, e, e), t);
+}
+
 // (row, col) of the e2-th lower-triangle entry. The estimate uses an FP32 square root (the
 // FP64 pipe is the bottleneck of the FP64 kernels) and integer fix-ups make it exact.
 __device__ __forceinline__ void lower_index(int e2, int& a, int& b) {
@@ -107,9 +125,9 @@ __global__ void __launch_bounds__(kThreads)
   const int ld = N + 1;
   R* A = dyn;          // [N][ld], lower triangle valid
   R* v = A + N * ld;   // [N]
-  R* w = v + N;        // [N]
+  R* w = v + N;        // [2][N]
   __shared__ R red[kWarps];
-  __shared__ R s_beta, s_kc;
+  __shared__ R s_beta;
   __shared__ int32_t s_zone;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (zset.none()) return;
@@ -147,26 +165,29 @@ __global__ void __launch_bounds__(kThreads)
     R* beta = ax + 2 * N;
     for (int k = 0; k < N - 2; k++) {
       const int L = N - k - 1;
-      if (warp == 0) {
+      // (another warp a block: the SM partitions' FP64 pipes share the reflectors' chains)
+      if (warp == (blockIdx.x & (kWarps - 1))) {
         // column k below the diagonal: x_i = A[k+1+i][k]
         R sig = 0;
-        for (int i = 1 + lane; i < L; i += 32) {
+        for (int i = lane; i < L; i += 32) {
           R x = A[(k + 1 + i) * ld + k];
-          sig = fma(x, x, sig);
+          v[i] = x;
+          if (i > 0) sig = fma(x, x, sig);
         }
         sig = warp_sum(sig);
         if (lane == 0) {
-          R x0 = A[(k + 1) * ld + k];
+          R x0 = v[0];
           R bk = 0;
-          const R mu = Prec<R>::sqrt_(x0 * x0 + sig);
+          const R mu = sqrt_of(x0 * x0 + sig);
           const R v0 = (x0 <= R(0)) ? x0 - mu : x0 + mu;  // v0 = x0 + sign(x0) mu
           const R vv = v0 * v0 + sig;
           if (sig == R(0) || !(vv > R(0)) || isinf(vv)) {  // nothing to annihilate
             e[k] = x0;
           } else {
             e[k] = (x0 <= R(0)) ? mu : -mu;               // alpha = -sign(x0) ||x||
-            bk = R(2) / vv;
+            bk = two_over(vv);
             A[(k + 1) * ld + k] = v0;
+            v[0] = v0;
           }
           d[k] = A[k * ld + k];
           beta[k] = bk;
@@ -175,27 +196,42 @@ __global__ void __launch_bounds__(kThreads)
       }
       __syncthreads();
       const R bk = s_beta;
-      if (bk == R(0)) continue;  // uniform across the block
-      for (int i = tid; i < L; i += kThreads) v[i] = A[(k + 1 + i) * ld + k];
-      __syncthreads();
-      // p = beta A22 v, one thread per row, A22 symmetric with its lower triangle stored
-      for (int i = tid; i < L; i += kThreads) {
-        const R* row = A + (k + 1 + i) * ld + (k + 1);
-        const R* col = A + (k + 1) * ld + (k + 1 + i);
-        R s = 0;
-        for (int j = 0; j < L; j++) s = fma((j <= i) ? row[j] : col[j * ld], v[j], s);
-        w[i] = bk * s;
+      if (bk == R(0)) {  // uniform across the block
+        __syncthreads();
+        continue;
       }
-      __syncthreads();
-      if (warp == 0) {
+      // A22 v, two threads a row (all four partitions' FP64 pipes down to the short rows), A22
+      // symmetric with its lower triangle stored; and v . (A22 v)
+      {
+        const int nw = (L + 31) >> 5;  // warps a half
+        const int part = warp < nw ? 0 : 1, i = tid - 32 * nw * part;
+        const int mid = (L + 1) >> 1, j1 = part ? L : mid;
         R pv = 0;
-        for (int i = lane; i < L; i += 32) pv = fma(w[i], v[i], pv);
-        pv = warp_sum(pv);
-        if (lane == 0) s_kc = R(0.5) * bk * pv;
+        if (warp < 2 * nw) {  // uniform in a warp
+          R s0 = 0, s1 = 0;
+          if (i < L) {
+            const R* row = A + (k + 1 + i) * ld + (k + 1);
+            const R* col = A + (k + 1) * ld + (k + 1 + i);
+            int j = part ? mid : 0;
+            for (; j + 1 < j1; j += 2) {
+              s0 = fma((j <= i) ? row[j] : col[j * ld], v[j], s0);
+              s1 = fma((j < i) ? row[j + 1] : col[(j + 1) * ld], v[j + 1], s1);
+            }
+            if (j < j1) s0 = fma((j <= i) ? row[j] : col[j * ld], v[j], s0);
+            s0 += s1;
+            w[part * N + i] = s0;
+            pv = s0 * v[i];
+          }
+          pv = warp_sum(pv);
+        }
+        if (lane == 0) red[warp] = pv;
       }
       __syncthreads();
-      const R Kc = s_kc;
-      for (int i = tid; i < L; i += kThreads) w[i] = fma(-Kc, v[i], w[i]);
+      if (32 * warp < L) {  // uniform in a warp
+        R pv = red[lane & (kWarps - 1)];
+        for (int o = kWarps / 2; o > 0; o >>= 1) pv += __shfl_xor_sync(0xffffffffu, pv, o);
+        if (tid < L) w[tid] = fma(-(R(0.5) * bk * bk * pv), v[tid], bk * (w[tid] + w[N + tid]));
+      }
       __syncthreads();
       // A22 -= v w^T + w v^T on the lower triangle
       const int E = L * (L + 1) / 2;
@@ -1074,7 +1110,7 @@ int grid_for_smem(const void* fn, size_t smem, int32_t nzc) {
 template <typename R>
 cudaError_t launch_e1(int N, int32_t nzc, R* d_GT, R* d_aux, ZoneSet zset, int32_t* d_work,
                       cudaStream_t st) {
-  size_t smem1 = (size_t)(N * (N + 1) + 2 * N) * sizeof(R);
+  size_t smem1 = (size_t)(N * (N + 1) + 3 * N) * sizeof(R);
   cudaError_t e = cudaFuncSetAttribute(k_eig_tridiag<R>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
   if (e != cudaSuccess) return e;
@@ -1112,7 +1148,7 @@ cudaError_t launch_e1<float>(int N, int32_t nzc, float* d_GT, float* d_aux, Zone
                              int32_t* d_work, cudaStream_t st) {
   if (N <= eig32_max_n()) return eig32_tridiag(N, nzc, d_GT, d_aux, zset.nobs, st);
   if (N <= eig128_max_n()) return eig128_tridiag(N, nzc, d_GT, d_aux, zset.nobs, st);
-  size_t smem1 = (size_t)(N * (N + 1) + 2 * N) * sizeof(float);
+  size_t smem1 = (size_t)(N * (N + 1) + 3 * N) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(k_eig_tridiag<float>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
   if (e != cudaSuccess) return e;
@@ -1249,6 +1285,31 @@ cudaError_t zone_eig_newton(int N, int32_t nzc, double* d_GT, const double* d_g,
   return cudaGetLastError();
 }
 
+// The FP64 transform without eigenvectors (zone_sqrt64.cu) and, for the zones out of its range,
+// the eigenvalue stages E2 and E3 on the same tridiagonal form.
+cudaError_t zone_eig_rational(int N, int32_t nzc, double* d_GT, const double* d_g,
+                              const int32_t* d_nobs, int rotate, double* d_ampl,
+                              int32_t* d_status, double* d_aux, double* d_Z, int32_t* d_work,
+                              cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(d_status, 0, sizeof(int32_t) * nzc, st);
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(d_work, 0, 4 * sizeof(int32_t), st);
+  if (e != cudaSuccess) return e;
+  e = launch_e1<double>(N, nzc, d_GT, d_aux, ZoneSet{d_nobs}, d_work, st);
+  int32_t* d_retries = d_work + 2;
+  if (e == cudaSuccess)
+    e = zone_sqrt64(N, nzc, d_GT, d_aux, aux_stride(N), d_g, d_nobs, rotate, d_ampl, d_status,
+                    d_work + 3, d_retries, st);
+  const ZoneSet zset{d_nobs, d_status, d_retries};
+  if (e == cudaSuccess) e = launch_e2<double>(N, nzc, d_aux, d_Z, zset, d_status, st);
+  if (e == cudaSuccess)
+    e = launch_e3<double>(N, nzc, d_GT, d_aux, d_Z, d_g, zset, rotate, d_ampl, d_status, d_work + 1,
+                          st);
+  if (e != cudaSuccess) return e;
+  count_launches(5);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 size_t zone_eig_aux(int N) { return (size_t)aux_stride(N); }
@@ -1265,6 +1326,12 @@ cudaError_t zone_eig_fp64(int N, int32_t nzc, double* d_GT, const double* d_g,
   if (tc_products && N >= kNewtonMinN && N <= isqrt_oz_max_n() && nzc > 1)
     return zone_eig_newton(N, nzc, d_GT, d_g, d_nobs, rotate, d_ampl, d_status, d_aux, d_Z, d_work,
                            st);
+  // wider ensembles, without eigenvectors (the eigensolve in 16,200 zones of 65 members 38 against
+  // 47 ms, of 80 58 against 76, of 100 101 against 181, of 128 235 against 405; 160 zones of 100
+  // members 2.1 against 13.1 ms). One zone as above
+  if (tc_products && N > isqrt_oz_max_n() && N <= sqrt64_max_n() && nzc > 1)
+    return zone_eig_rational(N, nzc, d_GT, d_g, d_nobs, rotate, d_ampl, d_status, d_aux, d_Z,
+                             d_work, st);
   return zone_eig_impl<double>(N, nzc, d_GT, d_g, d_nobs, rotate, d_ampl, d_status, d_aux, d_Z,
                                d_work, st, tc_products);
 }
