@@ -24,22 +24,29 @@ namespace {
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 16;
 
-__device__ __forceinline__ double warp_min(double x) {
-  for (int o = 16; o > 0; o >>= 1) x = fmin(x, __shfl_xor_sync(0xffffffffu, x, o));
-  return x;
-}
-__device__ __forceinline__ double warp_max(double x) {
-  for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
-  return x;
+// An FP64 value as a 64-bit integer of the same order (its own inverse on the bits).
+__device__ __forceinline__ long long order_key(long long b) {
+  return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFll);
 }
 
-// One block: min/max of u and v (v may be null).
+// One block: min/max of u and v (v may be null; NaNs are passed over). On integer keys: fmin and
+// fmax run at the FP64 pipe's two lanes a cycle, which for 64,800 values is 62 us of one SM's; so
+// 21 us.
 __global__ void __launch_bounds__(1024) k_bounds(const double* __restrict__ u, const double* __restrict__ v, int64_t m,
                          double* __restrict__ out) {
-  double umin = INFINITY, umax = -INFINITY, vmin = INFINITY, vmax = -INFINITY;
-  // eight loads of each in flight a thread: one block is bound by their latency (64,800 values:
-  // 62 us one at a time, 11 us so)
-  constexpr int kFly = 8;
+  const long long inf = __double_as_longlong(INFINITY);
+  long long lo[2], hi[2];
+#pragma unroll
+  for (int a = 0; a < 2; a++) lo[a] = order_key(inf), hi[a] = order_key(__double_as_longlong(-INFINITY));
+  if (!v) lo[1] = hi[1] = 0;
+  auto take = [&](int a, double x) {
+    const long long b = __double_as_longlong(x);
+    if ((b & 0x7FFFFFFFFFFFFFFFll) > inf) return;
+    const long long k = order_key(b);
+    lo[a] = min(lo[a], k);
+    hi[a] = max(hi[a], k);
+  };
+  constexpr int kFly = 4;  // loads of each in flight a thread
   for (int64_t j0 = threadIdx.x; j0 < m; j0 += kFly * (int64_t)blockDim.x) {
     double a[kFly], b[kFly];
 #pragma unroll
@@ -50,40 +57,36 @@ __global__ void __launch_bounds__(1024) k_bounds(const double* __restrict__ u, c
     }
 #pragma unroll
     for (int f = 0; f < kFly; f++) {
-      umin = fmin(umin, a[f]);
-      umax = fmax(umax, a[f]);
-      vmin = fmin(vmin, b[f]);
-      vmax = fmax(vmax, b[f]);
+      take(0, a[f]);
+      take(1, b[f]);
     }
   }
-  __shared__ double s[4][32];
-  umin = warp_min(umin);
-  umax = warp_max(umax);
-  vmin = warp_min(vmin);
-  vmax = warp_max(vmax);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  __shared__ long long s[4][32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  auto warp_reduce = [&]() {
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+      for (int o = 16; o > 0; o >>= 1) {
+        lo[a] = min(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+        hi[a] = max(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+      }
+  };
+  warp_reduce();
   if (l == 0) {
-    s[0][w] = umin;
-    s[1][w] = umax;
-    s[2][w] = vmin;
-    s[3][w] = vmax;
+#pragma unroll
+    for (int a = 0; a < 2; a++) s[2 * a][w] = lo[a], s[2 * a + 1][w] = hi[a];
   }
   __syncthreads();
   if (w == 0) {
-    int nw = blockDim.x >> 5;
-    umin = l < nw ? s[0][l] : INFINITY;
-    umax = l < nw ? s[1][l] : -INFINITY;
-    vmin = l < nw ? s[2][l] : INFINITY;
-    vmax = l < nw ? s[3][l] : -INFINITY;
-    umin = warp_min(umin);
-    umax = warp_max(umax);
-    vmin = warp_min(vmin);
-    vmax = warp_max(vmax);
+#pragma unroll
+    for (int a = 0; a < 2; a++) lo[a] = s[2 * a][l], hi[a] = s[2 * a + 1][l];  // (32 warps)
+    warp_reduce();
     if (l == 0) {
-      out[0] = umin;
-      out[1] = umax;
-      out[2] = vmin;
-      out[3] = vmax;
+#pragma unroll
+      for (int a = 0; a < 2; a++) {
+        out[2 * a] = __longlong_as_double(order_key(lo[a]));
+        out[2 * a + 1] = __longlong_as_double(order_key(hi[a]));
+      }
     }
   }
 }
@@ -111,8 +114,10 @@ __global__ void k_cell_id(CellGrid g, int64_t m, const double* __restrict__ u,
 
 // Exclusive scan of in[0..n) into out[0..n] (out[n] = total), one block, chunked with carry.
 // A chunk is kScanThreads x kScanItems values: thread t sums its kScanItems consecutive ones, the
-// sums are scanned by warp shuffles and one warp over the warps, with two barriers a chunk (64,800
-// values: 9 us; a log-step scan of 1,024 a chunk with twenty barriers took 114).
+// sums are scanned by warp shuffles and one warp over the warps, with two barriers a chunk; full
+// chunks of aligned arrays move 16 bytes at a time (one SM's stores bind it otherwise). 64,800
+// values: 27 us; 53 with single loads and stores; a log-step scan of 1,024 a chunk with twenty
+// barriers took 114.
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(kScanThreads) k_scan_single(const TI* __restrict__ in, int64_t n, TO* __restrict__ out,
                               int32_t* __restrict__ max_out) {
@@ -122,12 +127,25 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_single(const TI* __restri
   TO carry = 0;
   int32_t mymax = 0;
   int par = 0;
+  constexpr int kVi = 16 / sizeof(TI), kVo = 16 / sizeof(TO);  // values in 16 bytes
+  const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   for (int64_t base = 0; base < n; base += kScanThreads * kScanItems, par ^= 1) {
     const int64_t i0 = base + (int64_t)threadIdx.x * kScanItems;
-    TO x[kScanItems], sum = 0;
+    alignas(16) TI v[kScanItems];
+    alignas(16) TO x[kScanItems];
+    TO sum = 0;
+    const bool full = aligned && i0 + kScanItems <= n;
+    if (full) {
+#pragma unroll
+      for (int k = 0; k < kScanItems; k += kVi)
+        *reinterpret_cast<int4*>(v + k) = *reinterpret_cast<const int4*>(in + i0 + k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanItems; k++) v[k] = (i0 + k < n) ? in[i0 + k] : (TI)0;
+    }
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-      const TI a = (i0 + k < n) ? in[i0 + k] : (TI)0;
+      const TI a = v[k];
       if ((int32_t)a > mymax) mymax = (int32_t)a;
       x[k] = sum;
       sum += (TO)a;
@@ -154,8 +172,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_single(const TI* __restri
     __syncthreads();
     const TO off = carry + s[par][warp] + incl - sum;
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++)
-      if (i0 + k < n) out[i0 + k] = off + x[k];
+    for (int k = 0; k < kScanItems; k++) x[k] += off;
+    if (full) {
+#pragma unroll
+      for (int k = 0; k < kScanItems; k += kVo)
+        *reinterpret_cast<int4*>(out + i0 + k) = *reinterpret_cast<const int4*>(x + k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanItems; k++)
+        if (i0 + k < n) out[i0 + k] = x[k];
+    }
     carry += s[par][32];  // (the next chunk writes the other half)
   }
   if (threadIdx.x == 0) out[n] = carry;
