@@ -17,6 +17,7 @@
 // bind at 1.2 TFLOP/s; 1.33 GB and T's 2.1 GB take 0.5 ms), one zone of 324,000 rows 0.33 ms (2.21).
 // What bounds it: the staging and the read of the levels, which run one after the other in a CTA.
 #include <cuda_runtime.h>
+#include <math.h>
 
 #include "oakg_internal.cuh"
 #include "oz_slices.cuh"
@@ -39,6 +40,27 @@ struct UpdOz {
   static constexpr uint32_t kCols = 8 * RT;          // tensor-memory columns
 };
 
+// Rows with infinities or NaN have no fixed point; they get what the sum of their products is.
+__device__ __forceinline__ void mark_infinite(const double (&x)[8], int k0, unsigned long long* pos,
+                                              unsigned long long* neg) {
+#pragma unroll
+  for (int t = 0; t < 8; t++) {
+    const unsigned long long bit = 1ull << (k0 + t);
+    if (isnan(x[t]) || x[t] == INFINITY) atomicOr(pos, bit);
+    if (isnan(x[t]) || x[t] == -INFINITY) atomicOr(neg, bit);
+  }
+}
+__device__ __noinline__ double infinite_row(unsigned long long pos, unsigned long long neg,
+                                            const double* Tj, int N) {
+  double s = 0.0;
+  for (int k = 0; k < N; k++)
+    if (((pos | neg) >> k) & 1) {
+      const bool p = (pos >> k) & 1, n = (neg >> k) & 1;
+      s += (p && n ? NAN : (p ? INFINITY : -INFINITY)) * Tj[(int64_t)k * N];
+    }
+  return s;
+}
+
 template <int RT, typename S>
 __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
     k_zone_update_oz(int N, int32_t z0, int32_t nzc, int nsplit,
@@ -50,6 +72,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
   __shared__ __align__(16) double px[8][RT];
   __shared__ double am[64];
   __shared__ int32_t emT[64], emS[RT];
+  __shared__ unsigned long long s_inf[2][RT];  // a row's members at +inf, -inf (NaN: in both)
   __shared__ unsigned long long s_mbar;
   __shared__ uint32_t s_tmem;
   const uint32_t raw_addr = smem_u32(dyn_raw);
@@ -130,7 +153,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
       emT[tid] = 0;
       am[tid] = (tid < N) ? ampl[(int64_t)zl * N + tid] : 0.0;
     }
-    if (tid < RT) emS[tid] = 0;
+    if (tid < RT) emS[tid] = 0, s_inf[0][tid] = s_inf[1][tid] = 0;
     __syncthreads();
     auto top = [](const double (&x)[8]) {
       int e = 0;
@@ -142,7 +165,9 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
 #pragma unroll
     for (int u = 0; u < NU; u++) atomicMax(&emT[(tid + u * U::TT) & 63], top(tv[u]));
     for (int64_t tile = t0; tile < t1; tile++) {
-      atomicMax(&emS[sr], top(sv));
+      const int es = top(sv);
+      atomicMax(&emS[sr], es);
+      if (es == 0x7FF) mark_infinite(sv, 8 * sc, &s_inf[0][sr], &s_inf[1][sr]);
       double x = 0.0;
 #pragma unroll
       for (int t = 0; t < 8; t++) x = fma(sv[t], am[8 * sc + t], x);
@@ -222,13 +247,14 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
           const int r = 8 * gi + t;
           if (rt + r < i2) {
             double y = scaled_i64(v[t] + xch[r * 64 + j], emT[j] + emS[r] - 2 * 1022 - 57);
-            if (cbad || emS[r] == 0x7FF) y = __longlong_as_double(0x7FF8000000000000ll);
+            if (cbad) y = __longlong_as_double(0x7FF8000000000000ll);
+            else if (emS[r] == 0x7FF) y = infinite_row(s_inf[0][r], s_inf[1][r], Tz + j, N);
             Sa[rt + r + (int64_t)j * ldS] = (S)y;
           }
         }
       }
       __syncthreads();  // the exchange and the exponents are read
-      if (tid < RT) emS[tid] = 0;
+      if (tid < RT) emS[tid] = 0, s_inf[0][tid] = s_inf[1][tid] = 0;
       __syncthreads();
     }
   }

@@ -50,3 +50,18 @@ def test_float_storage_and_zones_without_observations():
     assert np.array_equal(a[1], b[1].astype(np.float32))
     rows = slice(45, 115)
     assert np.array_equal(b[1][rows], wide["Sf"][rows]) and np.array_equal(b[0][rows], wide["xf"][rows])
+
+
+def test_infinite_and_nan_rows():
+    """A row with an infinity or a NaN gets what the sum of its products is, and no other row does."""
+    p = _resized(_problem(64, 3, 6, lambda m, rng: rng.uniform(0.1, 1.0, m)), np.array([20, 70, 33]), 5)
+    Sf = p["Sf"]
+    Sf[3, 0], Sf[25, 63], Sf[30, [5, 40]], Sf[95, 17] = np.inf, -np.inf, (np.inf, -np.inf), np.nan
+    a = oak.loc_analysis(**p)
+    b = oak.loc_analysis(**p, simt_gram=True)
+    odd = [3, 25, 30, 95]
+    for x, y in ((a[0][odd], b[0][odd]), (a[1][odd], b[1][odd])):
+        assert not np.isfinite(x).any()
+        assert np.array_equal(x, y, equal_nan=True)
+    rest = np.setdiff1d(np.arange(Sf.shape[0]), odd)
+    assert np.isfinite(a[1][rest]).all() and np.isfinite(a[0][rest]).all()
