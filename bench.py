@@ -227,12 +227,13 @@ class ClockSampler:
 # --------------------------------------------------------------------------- GPU arm
 
 def algorithmic_work(c, nobs, stage):
-    """Algorithmic FP64 flops of one launch of a stage (per-zone counts x zones):
+    """Operations of one launch of a stage (per-zone counts x zones with observations):
     gram: p N (N+1) + 2 p N   (lower-triangular HS^T diag(c) HS plus HS^T diag(c) d)
-    eig:  9 N^3 (Householder tridiagonalisation + QR with vectors) + 2 N^3 + 4 N^2 (T, ampl),
-          less T_sym's N^2 (N+1) where it runs on the tensor cores (N <= 64): the count is
-          the FP64-pipe work, set against the FP64 peak
-    update: 2 nz N^2 + 2 nz N (Sf T and Sf ampl), zones with observations."""
+    eig:  17 to 64 members: the digit products of k_zone_isqrt_oz on the tensor cores, two
+          products (A Y, Y Z) of 34 digit pairs (levels 0..7) a residual, three residuals (two
+          Newton steps); else 9 N^3 (Householder tridiagonalisation + QR with vectors) +
+          2 N^3 + 4 N^2 (T, ampl) in FP64
+    update: 2 nz N^2 + 2 nz N (Sf T and Sf ampl)."""
     N = c.N
     act = nobs > 0
     p = nobs[act].astype(np.float64)
@@ -240,9 +241,19 @@ def algorithmic_work(c, nobs, stage):
     if stage == "gram":
         return float(np.sum(p * N * (N + 1) + 2 * p * N))
     if stage == "eig":
-        tsym_tc = float(N * N * (N + 1)) if N <= 64 else 0.0
-        return float(act.sum() * (11.0 * N ** 3 + 4.0 * N ** 2 - tsym_tc))
+        if 17 <= N <= 64:
+            return float(act.sum() * 3 * 2 * 34 * 2.0 * N ** 3)
+        return float(act.sum() * (11.0 * N ** 3 + 4.0 * N ** 2))
     return float(np.sum(2 * nz * N * N + 2 * nz * N))
+
+
+def tensor_peak():
+    """Measured dense 16-bit tensor rate in TFLOP/s (MEASURED_PEAKS.json), or the fallback."""
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            return float(json.load(f)["bf16_tflops"]), "measured cuBLAS bf16 GEMM on this GPU type"
+    except (OSError, KeyError, ValueError):
+        return 1900.0, "fallback: one earlier cuBLAS bf16 measurement"
 
 
 def main():
@@ -584,10 +595,14 @@ def main():
     per_step = {k: v / args.steps for k, v in stage_ms.items()}
     dom = max(("gram", "eig", "update"), key=lambda k: per_step[k])
     kernel = {"gram": "k_zone_gram_oz", "eig": "k_zone_eig_fp64",
-              "update": "k_zone_update_fp64"}[dom]
+              "update": "k_zone_update_oz"}[dom]
+    bound, peak, peak_source = ("fp64", peak_fp64.value,
+                                "measured FP64 FMA loop (oakg_fp64_peak) on this GPU")
+    if dom == "eig" and 17 <= c.N <= 64:
+        kernel, bound = "k_zone_isqrt_oz", "tensor"
+        peak, peak_source = tensor_peak()
     work = algorithmic_work(c, nobs, dom)
     achieved = work / (per_step[dom] / 1e3) / 1e12
-    peak = peak_fp64.value
     traffic = read_traffic(kernel)
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
@@ -607,12 +622,12 @@ def main():
         "graph": graph,
         "gpu_launches": int(launches),
         "stage_ms_per_step": per_step,
-        "roofline": {"kernel": kernel, "bound": "fp64", "achieved": achieved, "peak": peak,
+        "roofline": {"kernel": kernel, "bound": bound, "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak if peak > 0 else None,
-                     "peak_source": "measured FP64 FMA loop (oakg_fp64_peak) on this GPU",
-                     "kernels": ("E1-E4: k_eig_tridiag, k_eig_tridiag_values, "
-                                 "k_eig_vectors_fp64, k_eig_transform, k_zone_tsym_oz"
-                                 if kernel == "k_zone_eig_fp64" else kernel),
+                     "peak_source": peak_source,
+                     "kernels": ("k_eig_tridiag32, k_eig_values32, k_eig_vectors32, "
+                                 "k_eig_transform32, k_zone_isqrt_oz (the stage's time)"
+                                 if kernel == "k_zone_isqrt_oz" else kernel),
                      "traffic": traffic,
                      "algorithmic_flops_per_launch": work},
         "cpu_baseline": cpu,
