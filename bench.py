@@ -74,9 +74,9 @@ def dist_env():
 def workload_config(c, scale):
     return {"workload": c.name, "zones": int(c.Z), "n": int(c.n), "N": int(c.N), "m": int(c.m),
             "localisation": "Gaspari-Cohn locfun(d/6), maxLength 12 cells",
-            "precision": "fp64 (plain form: FP64 selection, weights, eigensolve and update; "
-                         "the Gram and the square-root transform's U (I+L)^-1/2 U^T as exact "
-                         "integer products of 8-bit slices on the BF16 tensor cores)",
+            "precision": "fp64 (plain form: FP64 selection and weights; the Gram, the Newton "
+                         "steps of the square-root transform and the update as exact integer "
+                         "products of 8-bit slices on the FP16 tensor cores)",
             "horizontal_scale": scale,
             "l2": "inputs larger than L2 (Sf and Sa 664 MB each at full scale)"}
 

@@ -32,12 +32,14 @@ __device__ __forceinline__ long long order_key(long long b) {
 // One block: min/max of u and v (v may be null; NaNs are passed over). On integer keys: fmin and
 // fmax run at the FP64 pipe's two lanes a cycle, which for 64,800 values is 62 us of one SM's; so
 // 21 us.
-__global__ void __launch_bounds__(1024) k_bounds(const double* __restrict__ u, const double* __restrict__ v, int64_t m,
-                         double* __restrict__ out) {
+__global__ void __launch_bounds__(1024)
+    k_bounds(const double* __restrict__ u, const double* __restrict__ v, int64_t m,
+             double* __restrict__ out) {
   const long long inf = __double_as_longlong(INFINITY);
   long long lo[2], hi[2];
 #pragma unroll
-  for (int a = 0; a < 2; a++) lo[a] = order_key(inf), hi[a] = order_key(__double_as_longlong(-INFINITY));
+  for (int a = 0; a < 2; a++)
+    lo[a] = order_key(inf), hi[a] = order_key(__double_as_longlong(-INFINITY));
   if (!v) lo[1] = hi[1] = 0;
   auto take = [&](int a, double x) {
     const long long b = __double_as_longlong(x);
@@ -119,8 +121,9 @@ __global__ void k_cell_id(CellGrid g, int64_t m, const double* __restrict__ u,
 // values: 27 us; 53 with single loads and stores; a log-step scan of 1,024 a chunk with twenty
 // barriers took 114.
 template <typename TI, typename TO>
-__global__ void __launch_bounds__(kScanThreads) k_scan_single(const TI* __restrict__ in, int64_t n, TO* __restrict__ out,
-                              int32_t* __restrict__ max_out) {
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_single(const TI* __restrict__ in, int64_t n, TO* __restrict__ out,
+                  int32_t* __restrict__ max_out) {
   __shared__ TO s[2][33];
   __shared__ int32_t smax[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -128,7 +131,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_single(const TI* __restri
   int32_t mymax = 0;
   int par = 0;
   constexpr int kVi = 16 / sizeof(TI), kVo = 16 / sizeof(TO);  // values in 16 bytes
-  const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  const bool aligned =
+      ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   for (int64_t base = 0; base < n; base += kScanThreads * kScanItems, par ^= 1) {
     const int64_t i0 = base + (int64_t)threadIdx.x * kScanItems;
     alignas(16) TI v[kScanItems];
