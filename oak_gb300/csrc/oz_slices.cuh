@@ -115,19 +115,23 @@ __device__ __forceinline__ void digit_pairs(unsigned long long a, unsigned long 
 }
 
 // vt 2^e2 rounded to nearest even, by integer operations (the conversion and scaling FP64
-// instructions avoided); |vt| < 2^63. Outside FP64's normal range the FP64 operations decide.
+// instructions avoided), over FP64's whole range; |vt| < 2^63.
 __device__ __forceinline__ double scaled_i64(long long vt, int e2) {
   if (vt == 0) return 0.0;
   const unsigned long long sgn = vt < 0 ? (1ull << 63) : 0ull;
   const unsigned long long m = vt < 0 ? (unsigned long long)(-vt) : (unsigned long long)vt;
   const int lz = __clzll((long long)m);
   const int be = 63 - lz + e2 + 1023;
-  if (be < 1 || be > 2045) {
-    int ex = e2 + 1023;
-    ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
-    return (double)vt * __longlong_as_double((long long)ex << 52);
-  }
   const unsigned long long mm = m << lz;  // leading one at bit 63
+  if (be < 1) {                           // subnormal: in units of 2^-1074
+    const int sh = 12 - be;
+    if (sh > 64) return __longlong_as_double((long long)sgn);
+    const unsigned long long q = sh < 64 ? mm >> sh : 0ull;
+    const unsigned long long rem = sh < 64 ? mm << (64 - sh) : mm, half = 1ull << 63;
+    return __longlong_as_double(
+        (long long)(sgn | (q + ((rem > half || (rem == half && (q & 1ull))) ? 1ull : 0ull))));
+  }
+  if (be > 2046) return __longlong_as_double((long long)(sgn | 0x7FF0000000000000ull));
   const unsigned long long mant = (mm >> 11) & 0xFFFFFFFFFFFFFull;
   const unsigned long long rem = mm & 0x7FFull;
   const unsigned long long up = (rem > 0x400ull || (rem == 0x400ull && (mant & 1ull))) ? 1ull : 0ull;
@@ -155,9 +159,12 @@ __device__ __forceinline__ void stage_digits(const long long (&F)[8], unsigned c
 template <int B>
 __device__ __forceinline__ long long fixed_of(double x, int E) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int e = (int)((b >> 52) & 0x7FFu);
-  if (e == 0) return 0;
-  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  int e = (int)((b >> 52) & 0x7FFu);
+  unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  if (e == 0) {  // a subnormal: no leading one
+    m ^= 0x10000000000000ull;
+    e = 1;
+  }
   const int s = e - 1075 + B - E;  // x 2^(B - E) = m 2^s
   unsigned long long F;
   if (s >= 0)
