@@ -59,7 +59,7 @@
 // zones with N = 64: 2.55 ms before, 2.13 ms now. Of about 95,000 cycles a zone 28,000 are staging, 25,000
 // accumulator reads, 24,000 selection and ranges, 10,000 FP64 weights. Reading the accumulators
 // every 8 K-tiles instead of 4 measured the same.
-// Every mbarrier wait is bounded; on expiry the kernel records ZST_TIMEOUT, stops taking
+// Every wait for the tensor core is bounded; on expiry the kernel records ZST_TIMEOUT, stops taking
 // zones, waits (bounded) for its MMAs and frees its tensor memory.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -103,7 +103,7 @@ struct OzShared {
   int32_t ring_e[kRing];             // and its biased exponent
   double ring_t[kRing];  // w^2 / r_q (yo - Hxf)_q
   OzZone zone[2];
-  unsigned long long done[2], full[2];  // a buffer's MMAs complete; its tile staged
+  unsigned long long done[2];           // a buffer's MMAs complete
   int32_t first[2];                     // the buffer's tile starts the accumulators
   int32_t warp_cnt[kThreads / 32];
   int32_t rlo[kThreads];   // first observation of each candidate range of a block of ranges
@@ -185,8 +185,20 @@ __device__ __forceinline__ void bar_workers() {
 __device__ __forceinline__ void bar_zone() {
   asm volatile("bar.sync 2, %0;" ::"n"(kThreads + 32) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+// buffer b's tile staged: the workers arrive, the issuer warp waits. A hardware barrier, as it waits
+// for the workers' progress: a run of zones that select nothing stages no tile, however long it is,
+// and only a wait for the tensor core may expire.
+__device__ __forceinline__ void tile_arrive(uint32_t b) {
+  if (b)
+    asm volatile("bar.arrive 4, %0;" ::"n"(kThreads + 32) : "memory");
+  else
+    asm volatile("bar.arrive 3, %0;" ::"n"(kThreads + 32) : "memory");
+}
+__device__ __forceinline__ void tile_wait(uint32_t b) {
+  if (b)
+    asm volatile("bar.sync 4, %0;" ::"n"(kThreads + 32) : "memory");
+  else
+    asm volatile("bar.sync 3, %0;" ::"n"(kThreads + 32) : "memory");
 }
 
 __global__ void __launch_bounds__(kThreads + 64, 1)
@@ -213,14 +225,11 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
   double* Gs = reinterpret_cast<double*>(tiles);  // and then the zone's G, [64][kLdG]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t done0 = smem_u32(&ts.done[0]), full0 = smem_u32(&ts.full[0]);
+  const uint32_t done0 = smem_u32(&ts.done[0]);
   if (tid == 0) {
 #pragma unroll
-    for (int b = 0; b < 2; b++) {
+    for (int b = 0; b < 2; b++)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(done0 + 8 * b));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full0 + 8 * b),
-                   "n"(kThreads / 32));
-    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     ts.stop = 0;
   }
@@ -247,16 +256,11 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
   if (warp == kThreads / 32) {
     // ---- issuer: every complete K-tile to the tensor core, so that no staging warp waits for the
     // tensor core's queue (28 MMAs a tile: p = 0, 2, 4, 6, [D_p ; D_(p+1)] by D_0 .. D_(7-p))
-    if (lane == 0) {
-      uint32_t phf[2] = {0u, 0u};
-      for (uint32_t n = 0;; n++) {
-        const uint32_t b = n & 1u;
-        if (!mbar_wait(full0 + 8 * b, phf[b])) {
-          late = true;
-          break;
-        }
-        phf[b] ^= 1u;
-        if (*(volatile int32_t*)&ts.stop) break;
+    for (uint32_t n = 0;; n++) {
+      const uint32_t b = n & 1u;
+      tile_wait(b);
+      if (*(volatile int32_t*)&ts.stop) break;
+      if (lane == 0) {
         const uint32_t acc0 = *(volatile int32_t*)&ts.first[b] ? 0u : 1u;
         fence_after();
         const uint32_t B = tile_addr + b * kBufBytes;
@@ -277,7 +281,6 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
         mma_commit(done0 + 8 * b);
       }
     }
-    __syncwarp();
   } else if (warp == kThreads / 32 + 1) {
     // ---- scout: picks the next zone and forms its FP64 set-up (divisions, floors: some 10,000
     // cycles on one thread) while the workers are at the present one
@@ -293,6 +296,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
           s.zl = zl;
           s.z = z;
           const double zx = zone_xyzt[4 * (int64_t)z + 0], zy = zone_xyzt[4 * (int64_t)z + 1];
+      __syncwarp();
           const double zzc = zone_xyzt[4 * (int64_t)z + 2], ztc = zone_xyzt[4 * (int64_t)z + 3];
           s.zu = (lp.loctype == 1) ? zx : (lp.loctype == 2 ? zzc : ztc);
           s.zv = (lp.loctype == 1) ? zy : 0.0;
@@ -505,7 +509,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
         fence_before();
         if (tid == 0) ts.first[b] = ctile == 0;
         __syncwarp();
-        if (lane == 0) mbar_arrive(full0 + 8 * b);
+        tile_arrive((uint32_t)b);
         pend[b] = true;
         nt++;
         ntile++;
@@ -731,7 +735,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
     if (tid == 0) ts.stop = 1;
     __syncwarp();
     bar_workers();
-    if (lane == 0) mbar_arrive(full0 + 8 * (nt & 1u));
+    tile_arrive(nt & 1u);
     if (abort) bar_zone();
     wait_done(0);
     wait_done(1);
