@@ -172,6 +172,10 @@ __device__ __forceinline__ long long fixed_row(unsigned long long m, int es, dou
   }
   const unsigned long long top = __umul64hi(m, mh);
   const unsigned long long F = (r < 64 && eh != 0) ? (top + (1ull << (r - 1))) >> r : 0ull;
+  if (F > (1ull << 54)) {
+    bad = 1;
+    return 0;
+  }
   return (hb >> 63) ? -(long long)F : (long long)F;
 }
 
