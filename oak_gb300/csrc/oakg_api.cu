@@ -993,17 +993,22 @@ int adjoint_impl(const oakg_dims* dims, const oakg_loc* loc, int32_t Z, const in
   if (N <= gram_oz_max_n() && m > 0 && !(lp.flags & OAKG_FLAG_SIMT_GRAM) &&
       (rc = scratch(c, B_OZSCR, gram_oz_scratch_bytes(m), &d_oz, "Gram exponents")))
     return rc;
-  cudaMemsetAsync(d_work + 2, 0, sizeof(int32_t), st);  // device status of the Gram
+  cudaMemsetAsync(d_work + 2, 0, 2 * sizeof(int32_t), st);  // device status, coarse zones
   cudaEventRecord(c->ev[1], st);
   for (int64_t k0 = 0; k0 < nact; k0 += chunk) {
     const int32_t nk = (int32_t)std::min<int64_t>(chunk, nact - k0);
-    // the forward's Gram (ZoneKernels<double>::gram) on the list
-    if (d_oz)
+    // the forward's Gram (ZoneKernels<double>::gram) on the list; in FP64 on all of it, or on the
+    // zones that the fixed point of the whole call's largest element would be too coarse for (the
+    // flags' memory is free: the list is made)
+    OzCoarse coarse;
+    if (d_oz) {
+      coarse = {d_flag + k0, d_work + 3};
       e = zone_gram_oz(P.g, P.so, m, N, lp, 0, nk, P.zxyzt, P.corr, P.maxl, d_G, d_gv, d_nobs,
-                       P.brute, d_work, d_work + 2, d_oz, st, nullptr, d_list + k0);
-    else
+                       P.brute, d_work, d_work + 2, d_oz, st, nullptr, d_list + k0, coarse);
+    }
+    if (e == cudaSuccess)
       e = zone_gram_fp64_list(P.g, P.so, N, lp, d_list + k0, nk, P.zxyzt, P.corr, P.maxl, d_G,
-                              d_gv, d_nobs, P.brute, d_work, st);
+                              d_gv, d_nobs, P.brute, d_work, st, coarse);
     if (e != cudaSuccess) return cuda_fail(e, "selection/Gram kernel");
     e = zone_adjoint_fp64(P.g, P.so, N, lp, d_list + k0, nk, P.zxyzt, P.corr, P.maxl, P.zstart,
                           P.Sf, ldS, d_seed, inflation, d_G, d_gv, d_nobs, d_dyo, d_dr, d_scal,

@@ -91,10 +91,15 @@ cudaError_t zone_gram_tc(const CellGrid& g, const SortedObs& so, int N, LocParam
                          int brute, int32_t* d_work, int32_t* d_err, cudaStream_t st,
                          const int32_t* order = nullptr);
 // Plain form on the tensor cores (zone_gram_oz.cu), N <= gram_oz_max_n(): G as an exact
-// product of 8-bit slices of X = diag(|w| / sqrt(r)) HS_sel on BF16 tensor cores, combined in
+// product of 8-bit slices of X = diag(|w| / sqrt(r)) HS_sel on FP16 tensor cores, combined in
 // 64-bit integers and FP64; the same selection, weights and outputs as zone_gram_fp64. d_scratch:
 // gram_oz_scratch_bytes(m) of device memory (column exponents, r^-1/2). d_err receives
-// ZST_TIMEOUT (OR) if a bounded device wait expired.
+// ZST_TIMEOUT (OR) if a bounded device wait expired. coarse: where given, the slots of zones that
+// the call's fixed point holds less exactly than FP64 products would, or whose inputs are not
+// finite, are set to 1 (others to 0) and counted.
+struct OzCoarse {
+  int32_t *zone = nullptr, *count = nullptr;
+};
 int gram_oz_max_n();
 size_t gram_oz_scratch_bytes(int64_t m);
 // The FP64 square-root transform of zones [0, nzc) on the tensor cores, N <= gram_oz_max_n():
@@ -111,7 +116,8 @@ cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int 
                          const double* max_len, double* d_G, double* d_g, int32_t* d_nobs,
                          int brute, int32_t* d_work, int32_t* d_err, void* d_scratch,
                          cudaStream_t st, const int32_t* order = nullptr,
-                         const int32_t* zlist = nullptr);  // zlist: as zone_gram_fp64_list
+                         const int32_t* zlist = nullptr,  // as zone_gram_fp64_list
+                         OzCoarse coarse = {});
 // FP32 copy of count doubles (HS rows for the mixed form).
 cudaError_t rows_to_fp32(const double* src, float* dst, int64_t count, cudaStream_t st);
 // FP64 copy of count floats (observation vectors given in FP32 storage).
@@ -167,7 +173,7 @@ cudaError_t zone_gram_fp64_list(const CellGrid& g, const SortedObs& so, int N, L
                                 const int32_t* zlist, int32_t nzc, const double* zone_xyzt,
                                 const double* corr_len, const double* max_len, double* d_G,
                                 double* d_g, int32_t* d_nobs, int brute, int32_t* d_work,
-                                cudaStream_t st);
+                                cudaStream_t st, OzCoarse only = {});
 // Adjoint of the analysis mean for the zones in zlist (see zone_adjoint.cu).
 cudaError_t zone_adjoint_fp64(const CellGrid& g, const SortedObs& so, int N, LocParams lp,
                               const int32_t* zlist, int32_t nzc, const double* zone_xyzt,

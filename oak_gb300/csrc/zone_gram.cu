@@ -117,7 +117,8 @@ __global__ void __launch_bounds__(kThreads)
                 const double* __restrict__ zone_xyzt, const double* __restrict__ corr_len,
                 const double* __restrict__ max_len, R* __restrict__ G, R* __restrict__ gv,
                 int32_t* __restrict__ nobs, int brute, int CH, int32_t* __restrict__ work,
-                const int32_t* __restrict__ zlist, const int32_t* __restrict__ order, int nx) {
+                const int32_t* __restrict__ zlist, const int32_t* __restrict__ order, int nx,
+                OzCoarse only) {
   extern __shared__ __align__(16) unsigned char dyn_raw[];
   R* dyn = reinterpret_cast<R*>(dyn_raw);
   R* sh = dyn;            // [CH][N]
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(kThreads)
   R* sinn = st + CH * N;  // [CH]
   __shared__ ZoneShared zs;
 
+  if (only.zone && *only.count == 0) return;
   const int E = N * (N + 1) / 2;
   const int nent = E + N;
   int32_t ea[MAXE], eb[MAXE];
@@ -152,6 +154,10 @@ __global__ void __launch_bounds__(kThreads)
     const int32_t w = zs.zone;  // pick number; zone order[z0 + w] when a pick order is given
     if (w >= nzc) break;
     const int32_t zl = order ? order[z0 + w] : w;
+    if (only.zone && !only.zone[zl]) {  // uniform
+      __syncthreads();
+      continue;
+    }
     const int32_t z = zlist ? zlist[zl] : z0 + zl;
     const double zx = zone_xyzt[4 * (int64_t)z + 0], zy = zone_xyzt[4 * (int64_t)z + 1];
     const double zzc = zone_xyzt[4 * (int64_t)z + 2], ztc = zone_xyzt[4 * (int64_t)z + 3];
@@ -370,7 +376,7 @@ cudaError_t launch_zone(const CellGrid& g, const SortedObs& so, int N, LocParams
                         const double* max_len, R* d_G, R* d_g, int32_t* d_nobs,
                         int brute, int32_t* d_work, cudaStream_t st,
                         const int32_t* zlist = nullptr, const int32_t* order = nullptr,
-                        int nx = -1) {
+                        int nx = -1, OzCoarse only = {}) {
   int CH = chunk_rows(N);
   size_t smem = (size_t)(2 * CH * N + CH) * sizeof(R);
   cudaError_t e = cudaFuncSetAttribute(k_zone_gram<MAXE, R>,
@@ -389,7 +395,7 @@ cudaError_t launch_zone(const CellGrid& g, const SortedObs& so, int N, LocParams
   if (e != cudaSuccess) return e;
   k_zone_gram<MAXE, R><<<grid, kThreads, smem, st>>>(g, so, N, lp, z0, nzc, zone_xyzt, corr_len,
                                                       max_len, d_G, d_g, d_nobs, brute, CH,
-                                                      d_work, zlist, order, nx < 0 ? N : nx);
+                                                      d_work, zlist, order, nx < 0 ? N : nx, only);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -475,9 +481,9 @@ cudaError_t zone_gram_fp64_list(const CellGrid& g, const SortedObs& so, int N, L
                                 const int32_t* zlist, int32_t nzc, const double* zone_xyzt,
                                 const double* corr_len, const double* max_len, double* d_G,
                                 double* d_g, int32_t* d_nobs, int brute, int32_t* d_work,
-                                cudaStream_t st) {
+                                cudaStream_t st, OzCoarse only) {
   OAKG_GRAM_DISPATCH_T(launch_zone, double, g, so, N, lp, 0, nzc, zone_xyzt, corr_len, max_len,
-                       d_G, d_g, d_nobs, brute, d_work, st, zlist);
+                       d_G, d_g, d_nobs, brute, d_work, st, zlist, nullptr, -1, only);
 }
 
 cudaError_t global_gram_fp64(int64_t m, int N, const double* HSf, int64_t ldH,

@@ -179,6 +179,15 @@ __device__ __forceinline__ long long fixed_row(unsigned long long m, int es, dou
   return (hb >> 63) ? -(long long)F : (long long)F;
 }
 
+// A zone whose largest element is 2^lx in a call whose largest is 2^em holds its Gram matrix to about
+// 2^(em + lx - 54) an observation. Where that exceeds 2^(kCoarseBits - 54) of the larger of the zone's
+// own products (2^(2 lx)) and the identity that is added to them, FP64 products of the zone's rows
+// would be more exact, and a caller that asks for it has such zones marked (one observation with an
+// error variance of 1e-12 beside others of 1e-2 would cost them 17 bits). Ordinary data are within 2
+// bits: no zone of the 2,400 seeded ones of the adjoint over 64,800 zones is marked.
+constexpr int kCoarseBits = 4;
+constexpr int kNoExponent = -100000;  // of a call without a non-zero element
+
 // 64-bit-integer lower-triangle index of (row j, column c <= j)
 __device__ __forceinline__ int tri(int j) { return j * (j + 1) / 2; }
 
@@ -205,6 +214,8 @@ __device__ __forceinline__ void tile_wait(uint32_t b) {
     asm volatile("bar.sync 3, %0;" ::"n"(kThreads + 32) : "memory");
 }
 
+// kCoarse: mark the zones whose fixed point is too coarse for them (kCoarseBits)
+template <bool kCoarse>
 __global__ void __launch_bounds__(kThreads + 64, 1)
     k_zone_gram_oz(CellGrid g, SortedObs so, int N, LocParams lp, int32_t z0, int32_t nzc,
                    const double* __restrict__ zone_xyzt, const double* __restrict__ corr_len,
@@ -212,9 +223,11 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
                    const double* __restrict__ isr, double* __restrict__ G,
                    double* __restrict__ gv, int32_t* __restrict__ nobs, int brute,
                    int32_t* __restrict__ work, int32_t* __restrict__ err,
-                   const int32_t* __restrict__ order, const int32_t* __restrict__ zlist) {
+                   const int32_t* __restrict__ order, const int32_t* __restrict__ zlist,
+                   OzCoarse coarse) {
   extern __shared__ __align__(16) unsigned char dyn_raw[];
   __shared__ __align__(16) OzShared ts;
+  __shared__ unsigned long long s_used[kCoarse ? NB : 1];  // the zone's |F| of each member, or-ed
   const uint32_t raw_addr = smem_u32(dyn_raw);
   const uint32_t pad = ((raw_addr + 1023u) & ~1023u) - raw_addr;
   unsigned char* tiles = dyn_raw + pad;  // 2 x kBufBytes (7 slices and a zero slice), 1024-aligned
@@ -473,6 +486,8 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
         ts.nrel = 0;
         ts.bad = 0;
       }
+      if (kCoarse && tid < NB) s_used[tid] = 0ull;  // (barriers below come before its first use)
+      unsigned long long used = 0ull;
       int head = 0, tail = 0, ntile = 0, ctile = 0, nflush = 0, nrel_local = 0, bad = 0;
       double gsum = 0.0, gsum1 = 0.0;
 
@@ -501,6 +516,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
           const int idx = (head + 8 * kq + i) & (kRing - 1);
           const bool ok = 8 * kq + i < rows;
           F[i] = fixed_row(ok ? ts.ring_m[idx] : 0ull, ts.ring_e[idx], hv[i], Ea, bad);
+          if (kCoarse) used |= (unsigned long long)(F[i] < 0 ? -F[i] : F[i]);
           // the innovation projection (two accumulators: shorter FMA chains)
           const double tq = ok ? ts.ring_t[idx] : 0.0;
           if (i & 1)
@@ -707,10 +723,25 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
       for (int o = 16; o > 0; o >>= 1) nrel_local += __shfl_xor_sync(0xffffffffu, nrel_local, o);
       if (lane == 0) atomicAdd(&ts.nrel, nrel_local);
       if (bad) atomicOr(&ts.bad, 1);
+      if (kCoarse) atomicOr(&s_used[a], used);
       gpart[kq * NB + a] = gsum + gsum1;
       bar_workers();  // nrel, bad and the partials published
       const int nrel = ts.nrel;
       if (tid == 0) nobs[z] = nrel;
+      if (kCoarse && warp == 0) {
+        // 2^em bounds the call's elements, 2^lx the zone's (all rounded to zero: by half a unit)
+        const int em = col_exp[NB];
+        int lx = em - 54;
+        for (int c = lane; c < N; c += 32)
+          if (s_used[c]) lx = max(lx, ts.E[c] + 10 - __clzll((long long)s_used[c]));
+        lx = __reduce_max_sync(0xffffffffu, lx);
+        const bool c = nrel > 0 && (ts.bad || (em > kNoExponent &&
+                                               em + lx > kCoarseBits + max(0, 2 * lx)));
+        if (lane == 0) {
+          coarse.zone[zl] = c;
+          if (c) atomicAdd(coarse.count, 1);
+        }
+      }
       if (ctile > 0) flush(nflush == 0, true, ts.bad != 0);
       if (nrel > 0 && ntile > 0) {
         double* Gz = G + (int64_t)zl * N * N;
@@ -787,9 +818,9 @@ __global__ void k_oz_colmax(int64_t m, int N, const double* __restrict__ HSt,
 
 __global__ void k_oz_exponents(int N, const unsigned long long* __restrict__ mx,
                                int32_t* __restrict__ E) {
-  const int a = threadIdx.x;
-  if (a >= N) return;
-  const double vmax = __longlong_as_double((long long)mx[a]);
+  const int a = threadIdx.x;  // NB threads
+  __shared__ int top[NB / 32];
+  const double vmax = a < N ? __longlong_as_double((long long)mx[a]) : 0.0;
   int e;
   if (vmax == 0.0) {
     e = 0;  // an all-zero column (or no usable observation)
@@ -803,7 +834,12 @@ __global__ void k_oz_exponents(int N, const unsigned long long* __restrict__ mx,
       e = (be == 0) ? -1022 : be - 1022;
     }
   }
-  E[a] = e;
+  if (a < N) E[a] = e;
+  // the largest of all, at E[NB]
+  const int t = __reduce_max_sync(0xffffffffu, vmax == 0.0 ? kNoExponent : e);
+  if ((a & 31) == 0) top[a >> 5] = t;
+  __syncthreads();
+  if (a == 0) E[NB] = max(top[0], top[1]);
 }
 
 // ------------------------------------------------------------------ square-root transform
@@ -1129,18 +1165,19 @@ __global__ void __launch_bounds__(kThreads, 1)
 int gram_oz_max_n() { return NB; }
 
 size_t gram_oz_scratch_bytes(int64_t m) {
-  return NB * sizeof(unsigned long long) + NB * sizeof(int32_t) + (size_t)m * sizeof(double);
+  return NB * sizeof(unsigned long long) + (NB + 2) * sizeof(int32_t) + (size_t)m * sizeof(double);
 }
 
 cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int N, LocParams lp,
                          int32_t z0, int32_t nzc, const double* zone_xyzt, const double* corr_len,
                          const double* max_len, double* d_G, double* d_g, int32_t* d_nobs,
                          int brute, int32_t* d_work, int32_t* d_err, void* d_scratch,
-                         cudaStream_t st, const int32_t* order, const int32_t* zlist) {
+                         cudaStream_t st, const int32_t* order, const int32_t* zlist,
+                         OzCoarse coarse) {
   if (N < 1 || N > NB || !so.HSt || !so.r || !d_scratch) return cudaErrorInvalidValue;
   unsigned long long* mx = reinterpret_cast<unsigned long long*>(d_scratch);
   int32_t* E = reinterpret_cast<int32_t*>(mx + NB);
-  double* isr = reinterpret_cast<double*>(E + NB);  // 8-byte aligned: NB int32 = 256 bytes
+  double* isr = reinterpret_cast<double*>(E + NB + 2);  // 8-byte aligned: E's 66 int32 are 264 bytes
   cudaError_t e = cudaMemsetAsync(mx, 0, NB * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 0;
@@ -1155,10 +1192,10 @@ cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int 
   }
   k_oz_exponents<<<1, NB, 0, st>>>(N, mx, E);
   count_launches(1);
-  e = cudaFuncSetAttribute(k_zone_gram_oz, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kDynSmem);
+  const auto kernel = coarse.zone ? k_zone_gram_oz<true> : k_zone_gram_oz<false>;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynSmem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_zone_gram_oz, cudaFuncAttributePreferredSharedMemoryCarveout,
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                            (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   // the shared-memory size admits one CTA per SM (it holds all 512 tensor-memory columns)
@@ -1166,9 +1203,9 @@ cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int 
   if (grid > nzc) grid = nzc > 0 ? nzc : 1;
   e = cudaMemsetAsync(d_work, 0, sizeof(int32_t), st);
   if (e != cudaSuccess) return e;
-  k_zone_gram_oz<<<grid, kThreads + 64, kDynSmem, st>>>(g, so, N, lp, z0, nzc, zone_xyzt, corr_len,
-                                                   max_len, E, isr, d_G, d_g, d_nobs, brute,
-                                                   d_work, d_err, order, zlist);
+  kernel<<<grid, kThreads + 64, kDynSmem, st>>>(g, so, N, lp, z0, nzc, zone_xyzt, corr_len, max_len, E,
+                                                isr, d_G, d_g, d_nobs, brute, d_work, d_err, order,
+                                                zlist, coarse);
   count_launches(1);
   return cudaGetLastError();
 }
