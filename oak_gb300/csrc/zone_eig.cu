@@ -88,24 +88,6 @@ __device__ __forceinline__ R warp_sum(R x) {
   return x;
 }
 
-// sqrt(x) and 2 / x: FP64 inside FP32's range from the FP32 value by the series of
-// (1 - e)^(-1/2) and 1 / (1 - e) to the second order (e below 2^-20: five and three FP64
-// operations on the chain of every reflector)
-__device__ __forceinline__ float sqrt_of(float x) { return sqrtf(x); }
-__device__ __forceinline__ double sqrt_of(double x) {
-  const float f = (float)x;
-  if (!(f > 1e-30f && f < 1e30f)) return sqrt(x);
-  const double r = (double)rsqrtf(f), t = x * r, e = fma(-t, r, 1.0);
-  return fma(t * e, fma(e, 0.375, 0.5), t);
-}
-__device__ __forceinline__ float two_over(float x) { return 2.f / x; }
-__device__ __forceinline__ double two_over(double x) {
-  const float f = (float)x;
-  if (!(f > 1e-30f && f < 1e30f)) return 2.0 / x;
-  const double r = (double)__fdividef(1.f, f), e = fma(-x, r, 1.0), t = 2.0 * r;
-  return fma(t, fma(e, e, e), t);
-}
-
 // (row, col) of the e2-th lower-triangle entry. The estimate uses an FP32 square root (the
 // FP64 pipe is the bottleneck of the FP64 kernels) and integer fix-ups make it exact.
 __device__ __forceinline__ void lower_index(int e2, int& a, int& b) {
@@ -178,14 +160,14 @@ __global__ void __launch_bounds__(kThreads)
         if (lane == 0) {
           R x0 = v[0];
           R bk = 0;
-          const R mu = sqrt_of(x0 * x0 + sig);
+          const R mu = Prec<R>::sqrt_(x0 * x0 + sig);
           const R v0 = (x0 <= R(0)) ? x0 - mu : x0 + mu;  // v0 = x0 + sign(x0) mu
           const R vv = v0 * v0 + sig;
           if (sig == R(0) || !(vv > R(0)) || isinf(vv)) {  // nothing to annihilate
             e[k] = x0;
           } else {
             e[k] = (x0 <= R(0)) ? mu : -mu;               // alpha = -sign(x0) ||x||
-            bk = two_over(vv);
+            bk = R(2) / vv;
             A[(k + 1) * ld + k] = v0;
             v[0] = v0;
           }

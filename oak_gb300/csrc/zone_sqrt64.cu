@@ -73,7 +73,9 @@ __device__ __forceinline__ double warp_sum(double x) {
 }
 
 // q / x for x in FP32's normal range: an FP32 reciprocal r and the series of 1 / (1 - e),
-// e = 1 - x r (below 2^-22), to the second order
+// e = 1 - x r (below 2^-21: x's rounding to FP32 and two units of the reciprocal), to the second
+// order. e is exact to 2^-53 of itself and the series' remainder is below 2^-63, so the roundings of
+// q r and of the last multiply-add are what is left: within 2^-52 of the quotient.
 __device__ __forceinline__ double quot(double q, double x) {
   const double r = (double)__fdividef(1.f, (float)x);
   const double e = fma(-x, r, 1.0);
