@@ -107,10 +107,11 @@ size_t gram_oz_scratch_bytes(int64_t m);
 // then T = T_sym Omega (rotate) in FP64, written to d_GT (N x N a zone). Inputs left by the
 // eigensolve's transform stage: the eigenvectors vector-major in d_Z (d_Z[k N + a] = U_ak),
 // q_k at d_aux[4N + k] and v at d_aux[k] of each zone (zone_eig_aux(N) elements a zone).
-// A bounded wait that expires sets ZST_TIMEOUT in the zone's d_status.
+// A bounded wait that expires sets ZST_TIMEOUT in the zone's d_status. d_retries: where given, only
+// the zones marked ZST_RETRY, *d_retries of them, whose mark is taken off.
 cudaError_t zone_tsym_oz(int N, int32_t nzc, double* d_GT, const double* d_aux,
                          const double* d_Z, const int32_t* d_nobs, int rotate,
-                         int32_t* d_status, cudaStream_t st);
+                         int32_t* d_status, cudaStream_t st, const int32_t* d_retries = nullptr);
 cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int N, LocParams lp,
                          int32_t z0, int32_t nzc, const double* zone_xyzt, const double* corr_len,
                          const double* max_len, double* d_G, double* d_g, int32_t* d_nobs,
@@ -206,9 +207,9 @@ cudaError_t zone_eig_fp32(int N, int32_t nzc, float* d_GT, const float* d_g,
                           float* d_aux, float* d_Z, int32_t* d_work, cudaStream_t st);
 size_t zone_eig_aux(int N);
 // ---- zone_isqrt_oz.cu: T = A^(-1/2) Omega and ampl = A^-1 g (A = I + G, G in d_GT, replaced by T)
-// of zones [0, nzc) with nobs > 0, N <= isqrt_oz_max_n(), from FP32 eigenpairs of G: vectors
+// of zones [0, nzc) with d_nobs[zl] != 0, N <= isqrt_oz_max_n(), from FP32 eigenpairs of G: vectors
 // vector-major in d_V (N x N a zone), eigenvalues at d_aux32[3N + k] (zone_eig_aux(N) a zone).
-// Sets each zone's d_status: 0, ZST_NAN, ZST_TIMEOUT, or ZST_RETRY (counted in *d_retries) with G
+// Sets each such zone's d_status: 0, ZST_NAN, ZST_TIMEOUT, or ZST_RETRY (counted in *d_retries) with G
 // left as it was where the eigenpairs were no start.
 int isqrt_oz_max_n();
 cudaError_t zone_isqrt_oz(int N, int32_t nzc, double* d_GT, const float* d_V, const float* d_aux32,
@@ -238,11 +239,21 @@ cudaError_t zone_eig_refine(int N, int32_t nzc, const float* d_G0, float* d_Z, f
 int eig32_max_n();
 cudaError_t eig32_tridiag(int N, int32_t nzc, float* d_GT, float* d_aux, const int32_t* d_nobs,
                           cudaStream_t st);
+// Zones that the Newton transform may take: mask (one element a zone, written by eig32_tridiag_of) is 0
+// for zones without observations and for those out of its reach, which are marked ZST_RETRY in
+// status and counted in *retries.
+struct NewtonReach {
+  int32_t *mask = nullptr, *status = nullptr, *retries = nullptr;
+  __device__ void leave(int32_t zl) const {
+    status[zl] = ZST_RETRY;
+    atomicAdd(retries, 1);
+  }
+};
 // the same on an FP64 matrix d_G (rounded to FP32, left as it is); the reflectors go to d_GT
 cudaError_t eig32_tridiag_of(int N, int32_t nzc, const double* d_G, float* d_GT, float* d_aux,
-                             const int32_t* d_nobs, cudaStream_t st);
+                             const int32_t* d_nobs, NewtonReach reach, cudaStream_t st);
 cudaError_t eig32_values(int N, int32_t nzc, float* d_aux, const int32_t* d_nobs,
-                         int32_t* d_status, cudaStream_t st);
+                         int32_t* d_status, cudaStream_t st, NewtonReach reach = {});
 cudaError_t eig32_vectors(int N, int32_t nzc, const float* d_aux, float* d_Z,
                           const int32_t* d_nobs, cudaStream_t st);
 cudaError_t eig32_transform(int N, int32_t nzc, float* d_GT, const float* d_aux, float* d_Z,

@@ -1001,7 +1001,7 @@ __global__ void __launch_bounds__(kThreads)
         ax[4 * N + i] = qs[i];
         ax[i] = rotate ? vv[i] : R(0);
       }
-      if (tid == 0) status[zl] = (status[zl] & ~ZST_RETRY) | (nan_flag ? ZST_NAN : 0);
+      if (tid == 0 && nan_flag) status[zl] |= ZST_NAN;  // (a retry's mark: zone_tsym_oz takes it off)
       __syncthreads();
       continue;
     }
@@ -1233,8 +1233,8 @@ cudaError_t zone_eig_impl(int N, int32_t nzc, R* d_GT, const R* d_g, const int32
   return cudaGetLastError();
 }
 
-// The FP64 transform from FP32 eigenpairs (zone_isqrt_oz.cu) and, for the zones whose Newton
-// iteration did not take, the FP64 stages E1-E3. The FP32 stages' matrices, vectors and aux live
+// The FP64 transform from FP32 eigenpairs (zone_isqrt_oz.cu) and, for the zones out of the Newton
+// iteration's reach or that it did not take, the FP64 stages E1-E4. The FP32 stages' matrices, vectors and aux live
 // in the FP64 scratch (d_Z: the reflectors, then the vectors; d_aux), which the FP64 stages
 // overwrite afterwards.
 cudaError_t zone_eig_newton(int N, int32_t nzc, double* d_GT, const double* d_g,
@@ -1247,21 +1247,24 @@ cudaError_t zone_eig_newton(int N, int32_t nzc, double* d_GT, const double* d_g,
   float* GT32 = reinterpret_cast<float*>(d_Z);
   float* V32 = GT32 + (size_t)nzc * N * N;
   float* aux32 = reinterpret_cast<float*>(d_aux);
-  e = eig32_tridiag_of(N, nzc, d_GT, GT32, aux32, d_nobs, st);
-  if (e == cudaSuccess) e = eig32_values(N, nzc, aux32, d_nobs, d_status, st);
-  if (e == cudaSuccess) e = eig32_vectors(N, nzc, aux32, V32, d_nobs, st);
-  if (e == cudaSuccess)
-    e = eig32_transform(N, nzc, GT32, aux32, V32, nullptr, d_nobs, rotate, nullptr, d_status, st, 1);
+  int32_t* mask = reinterpret_cast<int32_t*>(aux32 + (size_t)nzc * aux_stride(N));  // (d_aux's rest)
   int32_t* d_retries = d_work + 2;
+  const NewtonReach reach{mask, d_status, d_retries};
+  e = eig32_tridiag_of(N, nzc, d_GT, GT32, aux32, d_nobs, reach, st);
+  if (e == cudaSuccess) e = eig32_values(N, nzc, aux32, mask, d_status, st, reach);
+  if (e == cudaSuccess) e = eig32_vectors(N, nzc, aux32, V32, mask, st);
   if (e == cudaSuccess)
-    e = zone_isqrt_oz(N, nzc, d_GT, V32, aux32, d_g, d_nobs, rotate, d_ampl, d_status, d_retries,
-                      st);
+    e = eig32_transform(N, nzc, GT32, aux32, V32, nullptr, mask, rotate, nullptr, d_status, st, 1);
+  if (e == cudaSuccess)
+    e = zone_isqrt_oz(N, nzc, d_GT, V32, aux32, d_g, mask, rotate, d_ampl, d_status, d_retries, st);
   const ZoneSet zset{d_nobs, d_status, d_retries};
   if (e == cudaSuccess) e = launch_e1<double>(N, nzc, d_GT, d_aux, zset, d_work, st);
   if (e == cudaSuccess) e = launch_e2<double>(N, nzc, d_aux, d_Z, zset, d_status, st);
   if (e == cudaSuccess)
     e = launch_e3<double>(N, nzc, d_GT, d_aux, d_Z, d_g, zset, rotate, d_ampl, d_status, d_work + 1,
-                          st);
+                          st, 1);
+  if (e == cudaSuccess)
+    e = zone_tsym_oz(N, nzc, d_GT, d_aux, d_Z, d_nobs, rotate, d_status, st, d_retries);
   if (e != cudaSuccess) return e;
   count_launches(8);
   return cudaGetLastError();

@@ -81,6 +81,13 @@ __device__ __forceinline__ float wsum(float x) {
 // 16-column groups lying entirely there are skipped, and the first row set is skipped once all
 // its rows are final (k >= 31).
 constexpr int kZpb = 4;
+// The Newton transform's reach (zone_isqrt_oz.cu): of 300 zones each with one dominant, linearly or
+// geometrically falling or two clustered eigenvalues beside zero ones it took all to 270 with
+// lambda_max from 10^5 to 10^6, 152 to none from 10^6 to 10^7 and 3 at most beyond; with all
+// eigenvalues alike nearly all up to 10^9. Zones beyond are left before their eigenvectors are
+// formed. 16,200 zones of 64 members with lambda_max ~ 10^10: 32.1 ms; 45.0 with the whole attempt.
+constexpr float kReachMax = 2e9f;     // element of G
+constexpr float kReachSpread = 4e6f;  // (1 + lambda_max) / (1 + lambda_min)
 
 // Reflector k of E1 from row k of the matrix, published in rowbuf by the lane that holds it:
 // every lane takes entries lane and lane + 32 (sum of squares by a warp reduction), so the
@@ -110,16 +117,21 @@ __device__ __forceinline__ float warp_reflector(const float* rowbuf, int k, int 
   return bk;
 }
 
-// src: the matrices (GT itself, or FP64 ones, rounded to FP32).
+// src: the matrices (GT itself, or FP64 ones, rounded to FP32). reach (with FP64 ones): zones beyond
+// kReachMax are left out.
 template <typename S>
 __global__ void __launch_bounds__(32 * kZpb, 3)
     k_eig_tridiag32(int N, int32_t nzc, const S* src, float* GT, float* __restrict__ aux,
-                    const int32_t* __restrict__ nobs) {
+                    const int32_t* __restrict__ nobs, NewtonReach reach) {
   __shared__ __align__(16) float vbuf_s[kZpb][NB];
   __shared__ __align__(16) float wbuf_s[kZpb][NB];
   const int lane = threadIdx.x & 31, wz = threadIdx.x >> 5;
   const int32_t zl = blockIdx.x * kZpb + wz;
-  if (zl >= nzc || nobs[zl] == 0) return;  // warp-uniform; only warp-level synchronisation
+  if (zl >= nzc) return;  // warp-uniform; only warp-level synchronisation
+  if (nobs[zl] == 0) {
+    if (reach.mask && lane == 0) reach.mask[zl] = 0;
+    return;
+  }
   float* vbuf = vbuf_s[wz];
   float* wbuf = wbuf_s[wz];
   float* Gz = GT + (int64_t)zl * N * N;
@@ -136,6 +148,14 @@ __global__ void __launch_bounds__(32 * kZpb, 3)
 #pragma unroll
   for (int c = 0; c < NB; c++) amax = fmaxf(amax, fmaxf(fabsf(a0[c]), fabsf(a1[c])));
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (reach.mask) {
+    const bool in = amax <= kReachMax;  // (the largest eigenvalue is above every element)
+    if (lane == 0) {
+      reach.mask[zl] = in;
+      if (!in) reach.leave(zl);
+    }
+    if (!in) return;
+  }
   float scale = amax;
   if (!(scale > 0.f) || isinf(scale)) scale = 1.f;
   const float iscale = 1.f / scale;
@@ -746,8 +766,8 @@ __global__ void __launch_bounds__(32 * kZpb3, 4)
 constexpr int kT2 = 64;
 
 __global__ void __launch_bounds__(kT2)
-    k_eig_values32(int N, int32_t nzc, float* __restrict__ aux, const int32_t* __restrict__ nobs,
-                   int32_t* __restrict__ status) {
+    k_eig_values32(int N, int32_t nzc, float* __restrict__ aux, const int32_t* nobs,
+                   int32_t* status, NewtonReach reach) {
   __shared__ float sd[NB * kT2], se[NB * kT2];  // element i of thread t at [i * kT2 + t]
   const int t = threadIdx.x;
   const int32_t zl = blockIdx.x * kT2 + t;
@@ -856,6 +876,11 @@ __global__ void __launch_bounds__(kT2)
   }
   ax[5 * N + 1] = onenrm;
   if (st) status[zl] |= st;
+  if (reach.mask && 1.f + fmaxf(d[(N - 1) * kT2] * scale, 0.f) >
+                        kReachSpread * (1.f + fmaxf(d[0] * scale, 0.f))) {
+    reach.mask[zl] = 0;
+    reach.leave(zl);
+  }
 }
 
 // ------------------------------------------------------------------------------------ E2b
@@ -1552,9 +1577,9 @@ __global__ void __launch_bounds__(NB2, 3)
 int eig32_max_n() { return NB; }
 
 cudaError_t eig32_values(int N, int32_t nzc, float* d_aux, const int32_t* d_nobs,
-                         int32_t* d_status, cudaStream_t st) {
+                         int32_t* d_status, cudaStream_t st, NewtonReach reach) {
   if (N < 2 || N > NB) return cudaErrorInvalidValue;
-  k_eig_values32<<<(nzc + kT2 - 1) / kT2, kT2, 0, st>>>(N, nzc, d_aux, d_nobs, d_status);
+  k_eig_values32<<<(nzc + kT2 - 1) / kT2, kT2, 0, st>>>(N, nzc, d_aux, d_nobs, d_status, reach);
   return cudaGetLastError();
 }
 
@@ -1574,16 +1599,16 @@ cudaError_t eig32_tridiag(int N, int32_t nzc, float* d_GT, float* d_aux, const i
   if (N < 2 || N > NB) return cudaErrorInvalidValue;
   const int blocks = (nzc + kZpb - 1) / kZpb;
   k_eig_tridiag32<float><<<blocks > 0 ? blocks : 1, 32 * kZpb, 0, st>>>(N, nzc, d_GT, d_GT, d_aux,
-                                                                        d_nobs);
+                                                                        d_nobs, NewtonReach{});
   return cudaGetLastError();
 }
 
 cudaError_t eig32_tridiag_of(int N, int32_t nzc, const double* d_G, float* d_GT, float* d_aux,
-                             const int32_t* d_nobs, cudaStream_t st) {
+                             const int32_t* d_nobs, NewtonReach reach, cudaStream_t st) {
   if (N < 2 || N > NB) return cudaErrorInvalidValue;
   const int blocks = (nzc + kZpb - 1) / kZpb;
   k_eig_tridiag32<double><<<blocks > 0 ? blocks : 1, 32 * kZpb, 0, st>>>(N, nzc, d_G, d_GT, d_aux,
-                                                                         d_nobs);
+                                                                         d_nobs, reach);
   return cudaGetLastError();
 }
 

@@ -297,6 +297,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
         }
         mma_commit(done0 + 8 * b);
       }
+      __syncwarp();
     }
   } else if (warp == kThreads / 32 + 1) {
     // ---- scout: picks the next zone and forms its FP64 set-up (divisions, floors: some 10,000
@@ -313,7 +314,6 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
           s.zl = zl;
           s.z = z;
           const double zx = zone_xyzt[4 * (int64_t)z + 0], zy = zone_xyzt[4 * (int64_t)z + 1];
-      __syncwarp();
           const double zzc = zone_xyzt[4 * (int64_t)z + 2], ztc = zone_xyzt[4 * (int64_t)z + 3];
           s.zu = (lp.loctype == 1) ? zx : (lp.loctype == 2 ? zzc : ztc);
           s.zv = (lp.loctype == 1) ? zy : 0.0;
@@ -916,7 +916,8 @@ __device__ __forceinline__ void tmem_ld7x8(uint32_t ta, int c0, uint32_t (&r)[56
 __global__ void __launch_bounds__(kThreads, 1)
     k_zone_tsym_oz(int N, int32_t nzc, double* __restrict__ GT, const double* __restrict__ aux,
                    const double* __restrict__ Zg, const int32_t* __restrict__ nobs, int rotate,
-                   int32_t* __restrict__ status) {
+                   int32_t* status, const int32_t* __restrict__ retries) {
+  if (retries && *retries == 0) return;
   extern __shared__ __align__(16) unsigned char dyn_raw[];
   __shared__ __align__(16) TsShared ts;
   const uint32_t raw_addr = smem_u32(dyn_raw);
@@ -958,13 +959,16 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = ts.tmem_base;
   const double wv = 1.0 / sqrt((double)N);
   const double cw = 1.0 + wv, icw = 1.0 / cw;
-  const int nmine = (nzc - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  // this CTA's next zone from z on
+  auto next_zone = [&](int32_t z) {
+    while (z < nzc && (nobs[z] == 0 || (retries && !(status[z] & ZST_RETRY)))) z += gridDim.x;
+    return z;
+  };
   uint32_t ph = 0;
   bool pending = false;  // an MMA group whose completion was not observed (timeout)
 
-  // zone number i of this CTA's share into Upre / qpre / vpre (asynchronous copies)
-  auto prefetch = [&](int i) {
-    const int32_t zn = (int32_t)blockIdx.x + i * (int32_t)gridDim.x;
+  // zone zn into Upre / qpre / vpre (asynchronous copies)
+  auto prefetch = [&](int32_t zn) {
     const double* src = Zg + (int64_t)zn * N * N;
     for (int idx = tid; idx < N * N; idx += kThreads) cp_async8(Upre + idx, src + idx);
     const double* axn = aux + (int64_t)zn * (5 * N + 2);
@@ -1041,16 +1045,16 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   };
 
-  if (nmine > 0) {
-    prefetch(0);
+  int32_t zl = next_zone((int32_t)blockIdx.x), zn = nzc;  // in the accumulators; prefetched
+  if (zl < nzc) {
+    prefetch(zl);
     cp_async_wait_all();
     __syncthreads();
     stage_issue(0);
-    if (nmine > 1) prefetch(1);
+    zn = next_zone(zl + gridDim.x);
+    if (zn < nzc) prefetch(zn);
   }
-  for (int i = 0; i < nmine; i++) {
-    const int par = i & 1;
-    const int32_t zl = (int32_t)blockIdx.x + i * (int32_t)gridDim.x;
+  for (int par = 0; zl < nzc; par ^= 1) {
     if (tid == 0 && !mbar_wait(mbar, ph)) ts.flag = 1;
     ph ^= 1u;
     __syncthreads();  // MMA completion (or the timeout) published
@@ -1113,14 +1117,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int o = 16; o > 0; o >>= 1) sdot += __shfl_xor_sync(0xffffffffu, sdot, o);
       if (lane == 0) ts.uvuw = sdot;
     }
-    if (i + 1 < nmine) cp_async_wait_all();  // the next zone's copies (this thread's)
+    const int32_t znn = zn < nzc ? next_zone(zn + gridDim.x) : nzc;
+    if (zn < nzc) cp_async_wait_all();  // the next zone's copies (this thread's)
     fence_before();
     __syncthreads();  // T_sym, sums, u_v published; tensor memory read; next zone landed
-    if (i + 1 < nmine) {
+    if (zn < nzc) {
       stage_issue(par ^ 1);  // the next zone's MMAs run beside this zone's rotation
-      if (i + 2 < nmine) prefetch(i + 2);
+      if (znn < nzc) prefetch(znn);
     }
-    if (nobs[zl] == 0) continue;  // block-uniform: no T for a zone without observations
     double* Gz = GT + (int64_t)zl * N * N;
     if (rotate) {
       const double sgv = signbit(vv[N - 1]) ? -1.0 : 1.0;
@@ -1148,6 +1152,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         Gz[idx] = Ts[r * kTsLd + c];
       }
     }
+    if (retries && tid == 0) status[zl] &= ~ZST_RETRY;
+    zl = zn;
+    zn = znn;
   }
   // teardown: no MMA may still write tensor memory when it is freed, no copy still land
   cp_async_wait_all();
@@ -1212,7 +1219,7 @@ cudaError_t zone_gram_oz(const CellGrid& g, const SortedObs& so, int64_t m, int 
 
 cudaError_t zone_tsym_oz(int N, int32_t nzc, double* d_GT, const double* d_aux,
                          const double* d_Z, const int32_t* d_nobs, int rotate,
-                         int32_t* d_status, cudaStream_t st) {
+                         int32_t* d_status, cudaStream_t st, const int32_t* d_retries) {
   if (N < 1 || N > NB) return cudaErrorInvalidValue;
   if (nzc <= 0) return cudaSuccess;
   cudaError_t e = cudaFuncSetAttribute(k_zone_tsym_oz, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1226,7 +1233,7 @@ cudaError_t zone_tsym_oz(int N, int32_t nzc, double* d_GT, const double* d_aux,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = sms < nzc ? sms : nzc;
   k_zone_tsym_oz<<<grid, kThreads, kTsDynSmem, st>>>(N, nzc, d_GT, d_aux, d_Z, d_nobs, rotate,
-                                                     d_status);
+                                                     d_status, d_retries);
   count_launches(1);
   return cudaGetLastError();
 }
