@@ -19,6 +19,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <algorithm>
+
 #include "oakg_internal.cuh"
 #include "oz_slices.cuh"
 
@@ -63,7 +65,7 @@ __device__ __noinline__ double infinite_row(unsigned long long pos, unsigned lon
 
 template <int RT, typename S>
 __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
-    k_zone_update_oz(int N, int32_t z0, int32_t nzc, int nsplit,
+    k_zone_update_oz(int N, int32_t z0, int32_t nzc, int nranges,
                      const int64_t* __restrict__ zone_start, const S* xf, const S* Sf, int64_t ldS,
                      const double* __restrict__ T, const double* __restrict__ ampl,
                      const int32_t* __restrict__ nobs, S* xa, S* Sa, int32_t* __restrict__ err) {
@@ -108,15 +110,8 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
   uint32_t ph = 0;
   bool late = false, timeout = false;
 
-  const int64_t items = (int64_t)nzc * nsplit;
-  for (int64_t it = blockIdx.x; it < items && !timeout; it += gridDim.x) {
-    const int32_t zl = (int32_t)(it / nsplit);
-    const int part = (int)(it - (int64_t)zl * nsplit);
-    const int64_t i1 = zone_start[z0 + zl], i2 = zone_start[z0 + zl + 1];
-    // the part's tiles of RT rows
-    const int64_t tiles = (i2 - i1 + RT - 1) / RT;
-    const int64_t t0 = tiles * part / nsplit, t1 = tiles * (part + 1) / nsplit;
-    if (t0 >= t1) continue;  // uniform
+  // tiles [t0, t1) of zone zl, rows i1 .. i2 - 1
+  auto zone_tiles = [&](int32_t zl, int64_t i1, int64_t i2, int64_t t0, int64_t t1) {
     if (nobs[zl] == 0) {
       const int64_t r0 = i1 + t0 * RT, r1 = min(i1 + t1 * RT, i2);
       for (int64_t r = r0 + tid; r < r1; r += U::TT) xa[r] = xf[r];
@@ -124,7 +119,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
         for (int k = 0; k < N; k++)
           for (int64_t r = r0 + tid; r < r1; r += U::TT)
             Sa[r + (int64_t)k * ldS] = Sf[r + (int64_t)k * ldS];
-      continue;
+      return;
     }
     // T: unit (member column c, chunk of 8 k), k along the operand row; the first tile's rows beside
     constexpr int NU = 512 / U::TT;
@@ -193,7 +188,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
       fence_before();
       if (__syncthreads_or(late)) {
         timeout = true;
-        break;
+        return;
       }
       if (tid == 0) {
         fence_after();
@@ -257,6 +252,35 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
       if (tid < RT) emS[tid] = 0, s_inf[0][tid] = s_inf[1][tid] = 0;
       __syncthreads();
     }
+  };
+
+  // Work of the zones before zone z: their rows and, a zone, RT more (T's staging and the last
+  // tile's padding). A CTA takes equal ranges of it: a long zone's tiles fall into several ranges,
+  // short zones follow one another in one.
+  const int64_t first = zone_start[z0];
+  auto before = [&](int32_t z) { return zone_start[z0 + z] - first + (int64_t)RT * z; };
+  const int64_t total = before(nzc);
+  for (int range = blockIdx.x; range < nranges && !timeout; range += gridDim.x) {
+    const int64_t w0 = total * range / nranges, w1 = total * (range + 1) / nranges;
+    // the last zone that starts at or before w0, 32 pivots a step
+    int32_t zl = 0;
+    for (int32_t end = nzc; end - zl > 1;) {
+      const int32_t step = (end - zl + 31) >> 5, p = zl + lane * step;
+      const bool le = p < end && before(p) <= w0;
+      zl += (__popc(__ballot_sync(0xffffffffu, le)) - 1) * step;  // (lane 0's is)
+      end = min(end, zl + step);
+    }
+    for (; zl < nzc && !timeout; zl++) {
+      const int64_t b0 = before(zl), b1 = before(zl + 1);
+      if (b0 >= w1) break;
+      const int64_t i1 = zone_start[z0 + zl], i2 = zone_start[z0 + zl + 1];
+      const int64_t tiles = (i2 - i1 + RT - 1) / RT;
+      auto cut = [&](int64_t w) {
+        return w <= b0 ? 0 : (w >= b1 ? tiles : ((w - b0) * tiles + (b1 - b0 - 1)) / (b1 - b0));
+      };
+      const int64_t t0 = cut(w0), t1 = cut(w1);
+      if (t0 < t1) zone_tiles(zl, i1, i2, t0, t1);
+    }
   }
   // teardown: no MMA may still write tensor memory when it is freed
   if (__syncthreads_or(late) && tid == 0) {
@@ -287,13 +311,13 @@ cudaError_t launch(int N, int32_t z0, int32_t nzc, const int64_t* d_zone_start, 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t grid_max = (int64_t)sms * (RT == 32 ? 2 : 1);
-  // a long zone's tiles over several CTAs where the zones alone do not fill the chip
-  const int64_t tiles = (zone_max + RT - 1) / RT;
-  int64_t nsplit = (grid_max + nzc - 1) / nzc;
-  nsplit = nsplit < 1 ? 1 : (nsplit > tiles ? (tiles < 1 ? 1 : tiles) : nsplit);
-  const int64_t items = (int64_t)nzc * nsplit;
-  const int grid = (int)(items < grid_max ? items : grid_max);
-  k_zone_update_oz<RT, S><<<grid, U::TT, U::kSmem, st>>>(N, z0, nzc, (int)nsplit, d_zone_start, xf,
+  // Few zones: a range a CTA (no more than tiles). Many: as much work a range as one to four even
+  // zones have, so that even zones come in whole ones.
+  const int64_t tiles = std::max<int64_t>(1, (zone_max + RT - 1) / RT);
+  const int64_t per = std::min<int64_t>(4, std::max<int64_t>(1, nzc / (16 * grid_max)));
+  const int64_t nranges = nzc < grid_max ? std::min(nzc * tiles, grid_max) : (nzc + per - 1) / per;
+  const int grid = (int)std::min(nranges, grid_max);
+  k_zone_update_oz<RT, S><<<grid, U::TT, U::kSmem, st>>>(N, z0, nzc, (int)nranges, d_zone_start, xf,
                                                          Sf, ldS, d_T, d_ampl, d_nobs, xa, Sa, d_err);
   count_launches(1);
   return cudaGetLastError();
