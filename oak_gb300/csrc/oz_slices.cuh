@@ -139,19 +139,24 @@ __device__ __forceinline__ double scaled_i64(long long vt, int e2) {
 }
 
 // 8 consecutive K elements (54-bit fixed point) of an operand row as digit slices
-// of SLICE bytes
+// of SLICE bytes; false where seven digits do not hold one (from 2^55 - 2^47 units on)
 template <uint32_t SLICE>
-__device__ __forceinline__ void stage_digits(const long long (&F)[8], unsigned char* slices,
+__device__ __forceinline__ bool stage_digits(const long long (&F)[8], unsigned char* slices,
                                              uint32_t off) {
   uint32_t d[4][kDigits];
+  unsigned long long all = 0;
 #pragma unroll
-  for (int i = 0; i < 4; i++)
-    digit_pairs((unsigned long long)F[2 * i] + kDigitBias,
-                (unsigned long long)F[2 * i + 1] + kDigitBias, d[i]);
+  for (int i = 0; i < 4; i++) {
+    const unsigned long long a = (unsigned long long)F[2 * i] + kDigitBias,
+                             b = (unsigned long long)F[2 * i + 1] + kDigitBias;
+    all |= a | b;
+    digit_pairs(a, b, d[i]);
+  }
 #pragma unroll
   for (int p = 0; p < kDigits; p++)
     *reinterpret_cast<uint4*>(slices + p * SLICE + off) =
         make_uint4(d[0][p], d[1][p], d[2][p], d[3][p]);
+  return (all >> 56) == 0;  // the byte past the digits, 0xFF below -2^55
 }
 
 // round(x 2^(B - E)) for |x| < 2^E, B = 54 or 62, by integer operations: the 64-bit conversion

@@ -166,16 +166,13 @@ __device__ __forceinline__ long long fixed_row(unsigned long long m, int es, dou
   const unsigned long long mh = ((hb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 10;
   // s h 2^(54 - E) = P 2^-(2096 + E - es - eh), P = (m >> 11) (mh >> 10); top = P >> 43
   const int r = 2053 + E - es - eh;
-  if (eh == 0x7FF || (r < 7 && m != 0ull && eh != 0)) {  // non-finite, or above the bound
+  // non-finite, or above the bound (to 2^56 units: what seven digits do not hold, stage_digits finds)
+  if (eh == 0x7FF || (r < 7 && m != 0ull && eh != 0)) {
     bad = 1;
     return 0;
   }
   const unsigned long long top = __umul64hi(m, mh);
   const unsigned long long F = (r < 64 && eh != 0) ? (top + (1ull << (r - 1))) >> r : 0ull;
-  if (F > (1ull << 54)) {
-    bad = 1;
-    return 0;
-  }
   return (hb >> 63) ? -(long long)F : (long long)F;
 }
 
@@ -524,7 +521,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
           else
             gsum = fma(hv[i], tq, gsum);
         }
-        stage_digits<kSliceBytes>(F, tb, tile_off(a, kq));
+        if (!stage_digits<kSliceBytes>(F, tb, tile_off(a, kq))) bad = 1;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         fence_before();
         if (tid == 0) ts.first[b] = ctile == 0;

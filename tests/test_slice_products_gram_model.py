@@ -2,8 +2,9 @@
 oz_slices.cuh): the integer steps in Python integers and NumPy, against exact arithmetic.
 
 * fixed_row: the upper 64 bits of the significands' product shifted to the fixed point once, within
-  half a unit and 2^-9 of one (the truncated bits) of the exact value at every shift; products above
-  2^54 units and non-finite factors are flagged, zero and subnormal ones give 0.
+  half a unit and 2^-9 of one (the truncated bits) of the exact value at every shift; products of
+  2^56 units on and non-finite factors are flagged, zero and subnormal ones give 0.
+* stage_digits flags every value that seven digits do not hold, and no other.
 * digit_pairs: the FP16 numbers 0x6400 | byte less 1152 are the balanced base-256 digits.
 * The Gram over several accumulator reads: levels 0..7, even and odd first digits apart, levels 0..3
   and 4..7 (level 7 rounded to units of level 6 at each read of each half) as 64-bit integers, added
@@ -40,8 +41,6 @@ def fixed_row(m, es, h, E):
         return None
     top = (m * mh) >> 64
     F = ((top + (1 << (r - 1))) & M64) >> r if (r < 64 and eh != 0) else 0
-    if F > 1 << 54:
-        return None
     return -F if hb >> 63 else F
 
 
@@ -72,19 +71,19 @@ def test_fixed_row_rounds_once_at_every_shift():
         r = 2053 + E - es - ((_bits(h) >> 52) & 0x7FF)
         seen.add(r)
         if F is None:
-            assert abs(exact) > (1 << 54) - 1
+            assert abs(exact) >= 1 << 55
         else:
-            assert abs(F) <= 1 << 54 and abs(F - exact) <= Fraction(1, 2) + Fraction(1, 512)
+            assert abs(F) <= 1 << 56 and abs(F - exact) <= Fraction(1, 2) + Fraction(1, 512)
     assert {5, 6, 7, 8, 9, 62, 63, 64, 65} <= seen
 
 
 def test_fixed_row_flags_and_zeros():
     m, es = weight_parts(1.0)
     assert fixed_row(m, es, 1.0, 0) == 1 << 54
-    assert fixed_row(m, es, math.nextafter(1.0, 2.0), 0) is None      # r = 8, 2^54 + 4
-    assert fixed_row(m, es, 1.0 + 2.0 ** -50, 0) is None              # r = 8
-    assert fixed_row(m, es, 2.0, 0) is None                           # r = 7
-    assert fixed_row(m, es, 4.0, 0) is None                           # r = 6
+    assert fixed_row(m, es, math.nextafter(1.0, 2.0), 0) == (1 << 54) + 4
+    m2, es2 = weight_parts(1.5)
+    assert fixed_row(m2, es2, 1.5, 0) == 9 << 52  # r = 7, 2.25 times the bound
+    assert fixed_row(m, es, 2.0, 0) is None       # r = 6
     assert fixed_row(m, es, float("inf"), 0) is None and fixed_row(m, es, float("nan"), 0) is None
     assert fixed_row(*weight_parts(0.0), 1e300, 0) == 0
     assert fixed_row(m, es, 0.0, 0) == 0 and fixed_row(m, es, 5e-324, -1074 + 40) == 0
@@ -94,6 +93,18 @@ def test_digit_pairs_are_fp16_digits():
     byte = np.arange(256, dtype=np.uint16)
     h = (byte | np.uint16(0x6400)).view(np.float16) - np.uint16(0x6480).view(np.float16)
     assert np.array_equal(h.astype(int), byte.astype(int) - 128)
+
+
+def test_staged_digits_hold_the_value_or_flag_it():
+    edge = 0x7F7F7F7F7F7F7F  # seven digits of 127
+    rng = np.random.default_rng(6)
+    near = [s * (e + k) for s in (1, -1) for e in (edge, BIAS, 1 << 54, 1 << 55, 1 << 56) for k in
+            range(-3, 4)]
+    for F in near + [int(x) for x in rng.integers(-(1 << 57), 1 << 57, 3000)] + [0, 1 << 54]:
+        value = sum(d * 256 ** (6 - p) for p, d in enumerate(digits(F)))
+        held = ((F + BIAS) & M64) >> 56 == 0
+        assert held == (value == F)
+        assert held == (-BIAS <= F <= edge)
 
 
 def _halves(F, p_set, level):
