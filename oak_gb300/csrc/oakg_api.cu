@@ -291,6 +291,7 @@ struct ChunkArgs {
   // rows [HS_q | B_q] (m x (N + k))
   int smw_k = 0;
   const double* hst_aug = nullptr;
+  int64_t n = 0;  // rows of the state
   // host-memory pipeline: Sf (host) rows of each chunk copied into a.Sf on a copy stream, the
   // chunk's Sa / xa rows copied back to the host after its update (rows < n only); elements
   // are those of the state (double, or float with store32)
@@ -402,7 +403,7 @@ int run_chunks(Ctx* c, const ChunkArgs& a, int32_t** status_all, double* t_gram,
     } else {
       // plain form: Sa = Sf T on the tensor cores as exact slices, as the Gram
       const bool sa = a.store32 ? a.Sa32 != nullptr : a.Sa != nullptr;
-      if (!(a.lp.flags & OAKG_FLAG_SIMT_GRAM) && update_oz_pays(N, a.zone_max) && sa)
+      if (!(a.lp.flags & OAKG_FLAG_SIMT_GRAM) && update_oz_pays(N, a.n, a.Z) && sa)
         return a.store32 ? zone_update_oz(N, zz0, nq, a.zstart, a.zone_max, a.xf32, a.Sf32, a.ldS,
                                           T, za, nb, a.xa32, a.Sa32, *status_all, st)
                          : zone_update_oz(N, zz0, nq, a.zstart, a.zone_max, a.xf, a.Sf, a.ldS, T,
@@ -853,6 +854,7 @@ int locanalysis_impl(const oakg_dims* dims, const oakg_loc* loc, int32_t Z,
   int32_t* d_status_all = nullptr;
   ChunkArgs ca{P.g, P.so, lp, Z, N, ldS, P.zone_max, P.brute, all_ampl, P.zxyzt, P.corr, P.maxl,
                P.zstart, nullptr, nullptr, nullptr, nullptr, nullptr, d_nobs};
+  ca.n = n;
   if constexpr (f32) {
     ca.store32 = true;
     ca.xf32 = P.xf32;
@@ -1106,7 +1108,7 @@ int analysis_impl(const oakg_dims* dims, const double* xf, const double* Hxf,
   cudaEventRecord(c->ev[3], st);
   if (m == 0) cudaMemsetAsync(d_za, 0, N * sizeof(double), st);
   int32_t zone_max = (int32_t)std::min<int64_t>(n, INT32_MAX);
-  if (update_oz_pays(N, zone_max) && d_Sa)
+  if (update_oz_pays(N, n, 1) && d_Sa)
     e = zone_update_oz(N, 0, 1, d_zstart, zone_max, d_xf, d_Sf, ldS, d_G, d_za, d_nobs, d_xa, d_Sa,
                        d_status, st);
   else
@@ -1237,6 +1239,7 @@ int plan_create_impl(Plan** out, const oakg_dims* dims, const oakg_loc* loc, int
     pl->ca = ChunkArgs{pl->P.g, pl->P.so, lp, Z, N, dims->ldS, pl->P.zone_max, pl->P.brute,
                        all_ampl, pl->P.zxyzt, pl->P.corr, pl->P.maxl, pl->P.zstart, pl->P.xf,
                        pl->P.Sf, xa, Sa, ampl, d_nobs};
+    pl->ca.n = dims->n;
     pl->ca.refine = (lc->precision == OAKG_PREC_MIXED_FP64EIG);
     return OAKG_OK;
   };

@@ -333,11 +333,18 @@ cudaError_t write_amplitudes_fp32(int N, int32_t z0, int32_t nzc, const float* d
 // Sa = Sf T as exact slice products; Sa is required; S: double or float storage. d_err receives
 // ZST_TIMEOUT (OR) if a bounded device wait expired.
 int update_oz_max_n();
-// Whether it is the faster one: its cost does not fall with N (padded to 64), the CUDA-core
-// kernel's does with N^2. Zones of 20 rows (16,200): 0.71 ms against 1.40 at N = 64, 0.89 at 52,
-// 0.51 at 40; one zone of 324,000 rows: 0.33 ms against 2.21 at N = 64, 0.49 at 30.
-inline bool update_oz_pays(int N, int32_t zone_max) {
-  return N <= update_oz_max_n() && N >= (zone_max <= 32 ? 47 : 26);
+// Whether it is the faster one for n rows in Z zones: a zone costs it T's staging and its tiles of 32
+// rows whatever N (padded to 64), and the CUDA-core kernel about N^2 (rows + 4). Measured level, with
+// zones of 10 rows at 44 members, 15 at 37, 20 at 32, 26 at 28, 32 at 26 (one tile); 33 at 31, 40 at
+// 28, 64 at 23 (two); ahead at 1,000 rows from 26 on (below, not measured). 16,200 zones of 20 rows: 0.68 ms
+// against 2.33 at 64 members, 0.63 against 0.91 at 40, 0.59 against 0.42 at 26; of 1 row 0.55
+// against 0.42 at 64. The mean length decides: of zones that differ, the long ones cost both what
+// their rows cost.
+inline bool update_oz_pays(int N, int64_t n, int64_t Z) {
+  const double rows = Z > 0 ? (double)n / (double)Z : 0.0;
+  const double tiles = (double)(int64_t)((rows + 31.0) / 32.0);
+  return N <= update_oz_max_n() && N >= 26 &&
+         (double)N * N * (rows + 4.0) > 16e3 + 10e3 * tiles;
 }
 template <typename S>
 cudaError_t zone_update_oz(int N, int32_t z0, int32_t nzc, const int64_t* d_zone_start,

@@ -8,13 +8,16 @@
 // element of Sa is formed in units of 2^(E_c + F_r - 57) and rounded once to FP64. The mean is one
 // FP64 multiply-add an element.
 //
-// RT = 32 (zones of up to 32 rows): 256 threads and 256 tensor-memory columns, two CTAs an SM, one
-// staging while the other multiplies. RT = 64: 512 threads, one CTA an SM, a long zone's tiles
-// spread over several CTAs. Reads and writes are in place safe (a tile is read before it is
-// written; Sa may alias Sf, xa may alias xf). Every mbarrier wait is bounded (ZST_TIMEOUT).
+// RT = 32: 256 threads and 256 tensor-memory columns, two CTAs an SM, one staging while the other
+// multiplies. Tiles of 64 rows (512 threads, one CTA an SM) were never ahead: 16,200 zones of 20
+// rows 1.25 against 0.68 ms, of 64 rows 1.98 against 1.65, 5,000 of 1,000 rows 9.12 against 8.91,
+// one of 324,000 rows 0.33 against 0.27. Reads and writes are in place safe (a tile is read before
+// it is written; Sa may alias Sf, xa may alias xf). Every mbarrier wait is bounded (ZST_TIMEOUT).
+// Errors: 2^-54 of a row's largest element times a column's of T, an element, which T's own absolute
+// accuracy amounts to; an element of Sf far below its row's largest is not held to its own last bit.
 //
 // Measured, N = 64: 64,800 zones of 20 rows 2.85 ms (9.4 on the FP64 pipe, which its 2 n N^2 flops
-// bind at 1.2 TFLOP/s; 1.33 GB and T's 2.1 GB take 0.5 ms), one zone of 324,000 rows 0.33 ms (2.21).
+// bind at 1.2 TFLOP/s; 1.33 GB and T's 2.1 GB take 0.5 ms), one zone of 324,000 rows 0.27 ms (2.21).
 // What bounds it: the staging and the read of the levels, which run one after the other in a CTA.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -30,17 +33,16 @@ namespace {
 
 constexpr uint32_t kSliceT = 64u * 128u;  // a digit slice of T: 64 members
 
-template <int RT>
-struct UpdOz {
-  static constexpr int TT = 8 * RT;                  // threads
-  static constexpr uint32_t kSliceS = RT * 128u;     // a digit slice of RT state rows
-  static constexpr uint32_t kOffS = 8 * kSliceT;     // T: 7 digit slices and a zero slice
-  // the exchange of the two halves' sums overlays the rows' slices
-  static constexpr size_t kRows = 7 * (size_t)kSliceS;
-  static_assert(kRows >= 64 * RT * sizeof(long long), "exchange");
-  static constexpr size_t kSmem = 1024 + kOffS + kRows;
-  static constexpr uint32_t kCols = 8 * RT;          // tensor-memory columns
-};
+constexpr int RT = 32;                       // state rows a tile
+constexpr int TT = 8 * RT;                   // threads
+constexpr int kCtas = 2;                     // an SM
+constexpr uint32_t kSliceS = RT * 128u;      // a digit slice of RT state rows
+constexpr uint32_t kOffS = 8 * kSliceT;      // T: 7 digit slices and a zero slice
+// the exchange of the two halves' sums overlays the rows' slices
+constexpr size_t kRows = 7 * (size_t)kSliceS;
+static_assert(kRows >= 64 * RT * sizeof(long long), "exchange");
+constexpr size_t kSmem = 1024 + kOffS + kRows;
+constexpr uint32_t kCols = 8 * RT;           // tensor-memory columns
 
 // Rows with infinities or NaN have no fixed point; they get what the sum of their products is.
 __device__ __forceinline__ void mark_infinite(const double (&x)[8], int k0, unsigned long long* pos,
@@ -63,13 +65,12 @@ __device__ __noinline__ double infinite_row(unsigned long long pos, unsigned lon
   return s;
 }
 
-template <int RT, typename S>
-__global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
+template <typename S>
+__global__ void __launch_bounds__(TT, kCtas)
     k_zone_update_oz(int N, int32_t z0, int32_t nzc, int nranges,
                      const int64_t* __restrict__ zone_start, const S* xf, const S* Sf, int64_t ldS,
                      const double* __restrict__ T, const double* __restrict__ ampl,
                      const int32_t* __restrict__ nobs, S* xa, S* Sa, int32_t* __restrict__ err) {
-  using U = UpdOz<RT>;
   extern __shared__ __align__(16) unsigned char dyn_raw[];
   __shared__ __align__(16) double px[8][RT];
   __shared__ double am[64];
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
   const uint32_t pad = ((raw_addr + 1023u) & ~1023u) - raw_addr;
   unsigned char* sm = dyn_raw + pad;
   const uint32_t sa = raw_addr + pad;
-  long long* xch = reinterpret_cast<long long*>(sm + U::kOffS);  // [RT rows][64 members]
+  long long* xch = reinterpret_cast<long long*>(sm + kOffS);  // [RT rows][64 members]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // tensor-memory lane quarter q: members 32 (q & 1) .. + 31, odd digits for q >= 2; the thread
   // owns member j, state rows 8 gi .. 8 gi + 7 of the tile
@@ -94,12 +95,12 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (uint32_t i = tid; i < kSliceT / 16; i += U::TT)
+  for (uint32_t i = tid; i < kSliceT / 16; i += TT)
     reinterpret_cast<uint4*>(sm + 7 * kSliceT)[i] = make_uint4(0, 0, 0, 0);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&s_tmem)),
-                 "r"(U::kCols));
+                 "r"(kCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   fence_before();
@@ -114,20 +115,20 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
   auto zone_tiles = [&](int32_t zl, int64_t i1, int64_t i2, int64_t t0, int64_t t1) {
     if (nobs[zl] == 0) {
       const int64_t r0 = i1 + t0 * RT, r1 = min(i1 + t1 * RT, i2);
-      for (int64_t r = r0 + tid; r < r1; r += U::TT) xa[r] = xf[r];
+      for (int64_t r = r0 + tid; r < r1; r += TT) xa[r] = xf[r];
       if (Sa != Sf)
         for (int k = 0; k < N; k++)
-          for (int64_t r = r0 + tid; r < r1; r += U::TT)
+          for (int64_t r = r0 + tid; r < r1; r += TT)
             Sa[r + (int64_t)k * ldS] = Sf[r + (int64_t)k * ldS];
       return;
     }
     // T: unit (member column c, chunk of 8 k), k along the operand row; the first tile's rows beside
-    constexpr int NU = 512 / U::TT;
+    constexpr int NU = 512 / TT;
     double tv[NU][8], sv[8];
     const double* Tz = T + (int64_t)zl * N * N;
 #pragma unroll
     for (int u = 0; u < NU; u++) {
-      const int c = (tid + u * U::TT) & 63, ch = (tid + u * U::TT) >> 6;
+      const int c = (tid + u * TT) & 63, ch = (tid + u * TT) >> 6;
 #pragma unroll
       for (int t = 0; t < 8; t++) {
         const int k = 8 * ch + t;
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
       return e;
     };
 #pragma unroll
-    for (int u = 0; u < NU; u++) atomicMax(&emT[(tid + u * U::TT) & 63], top(tv[u]));
+    for (int u = 0; u < NU; u++) atomicMax(&emT[(tid + u * TT) & 63], top(tv[u]));
     for (int64_t tile = t0; tile < t1; tile++) {
       const int es = top(sv);
       atomicMax(&emS[sr], es);
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
       if (tile == t0) {
 #pragma unroll
         for (int u = 0; u < NU; u++) {
-          const int c = (tid + u * U::TT) & 63, ch = (tid + u * U::TT) >> 6;
+          const int c = (tid + u * TT) & 63, ch = (tid + u * TT) >> 6;
           long long F[8];
 #pragma unroll
           for (int t = 0; t < 8; t++) F[t] = fixed_of<54>(tv[u][t], emT[c] - 1022);
@@ -182,7 +183,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
         long long F[8];
 #pragma unroll
         for (int t = 0; t < 8; t++) F[t] = fixed_of<54>(sv[t], emS[sr] - 1022);
-        stage_digits<U::kSliceS>(F, sm + U::kOffS, tile_off(sr, sc));
+        stage_digits<kSliceS>(F, sm + kOffS, tile_off(sr, sc));
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       fence_before();
@@ -192,25 +193,17 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
       }
       if (tid == 0) {
         fence_after();
-        const uint32_t B = sa + U::kOffS;
+        const uint32_t B = sa + kOffS;
 #pragma unroll 1
         for (int kk = 0; kk < 4; kk++) {
           const uint32_t ko = kk * 32, acc = kk > 0 ? 1u : 0u;
           const uint64_t b0 = make_desc(B + ko);
           // D_p D_q, p even (odd in the upper half), in column block p + q
           uint64_t a = make_desc(sa + ko);
-          if (RT == 32) {
-            mma_f16(tmem, a, b0, idesc_f16(7 * RT), acc);                       // p = 0, q = 0..6
-            a = make_desc(sa + 2 * kSliceT + ko);
-            mma_f16(tmem + 2 * RT, a, b0, idesc_f16(5 * RT), 1u);               // p = 2, q = 0..4
-          } else {
-            mma_f16(tmem, a, b0, idesc_f16(4 * RT), acc);                       // p = 0, q = 0..3
-            mma_f16(tmem + 4 * RT, a, make_desc(B + 4 * U::kSliceS + ko), idesc_f16(3 * RT), acc);
-            a = make_desc(sa + 2 * kSliceT + ko);
-            mma_f16(tmem + 2 * RT, a, b0, idesc_f16(4 * RT), 1u);               // p = 2, q = 0..3
-            mma_f16(tmem + 6 * RT, a, make_desc(B + 4 * U::kSliceS + ko), idesc_f16(RT), 1u);
-          }
-          mma_f16(tmem + 7 * RT, a, make_desc(B + 5 * U::kSliceS + ko), idesc_f16(RT), acc);
+          mma_f16(tmem, a, b0, idesc_f16(7 * RT), acc);          // p = 0, q = 0..6
+          a = make_desc(sa + 2 * kSliceT + ko);
+          mma_f16(tmem + 2 * RT, a, b0, idesc_f16(5 * RT), 1u);  // p = 2, q = 0..4
+          mma_f16(tmem + 7 * RT, a, make_desc(B + 5 * kSliceS + ko), idesc_f16(RT), acc);
           mma_f16(tmem + 4 * RT, make_desc(sa + 4 * kSliceT + ko), b0, idesc_f16(4 * RT), 1u);
           mma_f16(tmem + 6 * RT, make_desc(sa + 6 * kSliceT + ko), b0, idesc_f16(2 * RT), 1u);
         }
@@ -292,35 +285,7 @@ __global__ void __launch_bounds__(8 * RT, RT == 32 ? 2 : 1)
   fence_after();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(U::kCols));
-}
-
-template <int RT, typename S>
-cudaError_t launch(int N, int32_t z0, int32_t nzc, const int64_t* d_zone_start, int32_t zone_max,
-                   const S* xf, const S* Sf, int64_t ldS, const double* d_T, const double* d_ampl,
-                   const int32_t* d_nobs, S* xa, S* Sa, int32_t* d_err, cudaStream_t st) {
-  using U = UpdOz<RT>;
-  cudaError_t e = cudaFuncSetAttribute(
-      k_zone_update_oz<RT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)U::kSmem);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_zone_update_oz<RT, S>,
-                           cudaFuncAttributePreferredSharedMemoryCarveout,
-                           (int)cudaSharedmemCarveoutMaxShared);
-  if (e != cudaSuccess) return e;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t grid_max = (int64_t)sms * (RT == 32 ? 2 : 1);
-  // Few zones: a range a CTA (no more than tiles). Many: as much work a range as one to four even
-  // zones have, so that even zones come in whole ones.
-  const int64_t tiles = std::max<int64_t>(1, (zone_max + RT - 1) / RT);
-  const int64_t per = std::min<int64_t>(4, std::max<int64_t>(1, nzc / (16 * grid_max)));
-  const int64_t nranges = nzc < grid_max ? std::min(nzc * tiles, grid_max) : (nzc + per - 1) / per;
-  const int grid = (int)std::min(nranges, grid_max);
-  k_zone_update_oz<RT, S><<<grid, U::TT, U::kSmem, st>>>(N, z0, nzc, (int)nranges, d_zone_start, xf,
-                                                         Sf, ldS, d_T, d_ampl, d_nobs, xa, Sa, d_err);
-  count_launches(1);
-  return cudaGetLastError();
+                 "r"(kCols));
 }
 
 }  // namespace
@@ -334,10 +299,26 @@ cudaError_t zone_update_oz(int N, int32_t z0, int32_t nzc, const int64_t* d_zone
                            S* Sa, int32_t* d_err, cudaStream_t st) {
   if (N < 1 || N > update_oz_max_n() || !Sa) return cudaErrorInvalidValue;
   if (nzc <= 0) return cudaSuccess;
-  return zone_max <= 32 ? launch<32, S>(N, z0, nzc, d_zone_start, zone_max, xf, Sf, ldS, d_T, d_ampl,
-                                        d_nobs, xa, Sa, d_err, st)
-                        : launch<64, S>(N, z0, nzc, d_zone_start, zone_max, xf, Sf, ldS, d_T, d_ampl,
-                                        d_nobs, xa, Sa, d_err, st);
+  cudaError_t e = cudaFuncSetAttribute(k_zone_update_oz<S>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_zone_update_oz<S>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                           (int)cudaSharedmemCarveoutMaxShared);
+  if (e != cudaSuccess) return e;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t grid_max = (int64_t)sms * kCtas;
+  // Few zones: a range a CTA (no more than tiles). Many: as much work a range as one to four even
+  // zones have, so that even zones come in whole ones.
+  const int64_t tiles = std::max<int64_t>(1, (zone_max + RT - 1) / RT);
+  const int64_t per = std::min<int64_t>(4, std::max<int64_t>(1, nzc / (16 * grid_max)));
+  const int64_t nranges = nzc < grid_max ? std::min(nzc * tiles, grid_max) : (nzc + per - 1) / per;
+  const int grid = (int)std::min(nranges, grid_max);
+  k_zone_update_oz<S><<<grid, TT, kSmem, st>>>(N, z0, nzc, (int)nranges, d_zone_start, xf, Sf, ldS,
+                                               d_T, d_ampl, d_nobs, xa, Sa, d_err);
+  count_launches(1);
+  return cudaGetLastError();
 }
 
 template cudaError_t zone_update_oz<double>(int, int32_t, int32_t, const int64_t*, int32_t,
