@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
             }
           }
           int incl = rlen;
-  #pragma unroll
+#pragma unroll
           for (int o = 1; o < 32; o <<= 1) {
             const int t = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += t;
@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
           if (warp == 0) {
             const int wsum = (lane < kThreads / 32) ? ts.warp_cnt[lane] : 0;
             int winc = wsum;
-  #pragma unroll
+#pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
               const int t = __shfl_up_sync(0xffffffffu, winc, o);
               if (lane >= o) winc += t;
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(kThreads + 64, 1)
           if (lane == 0) ts.warp_cnt[warp] = __popc(ball);
           bar_workers();
           int before = 0, total = 0;
-  #pragma unroll
+#pragma unroll
           for (int w2 = 0; w2 < kThreads / 32; w2++) {
             const int cnt = ts.warp_cnt[w2];
             before += (w2 < warp) ? cnt : 0;
