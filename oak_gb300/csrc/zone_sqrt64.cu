@@ -343,10 +343,25 @@ __global__ void __launch_bounds__(kThreads, 2)
       __syncthreads();
       return part[col] + part[kMaxN + col];
     };
-    if (tid < kMaxN) x0[tid] = tid < N ? gv[(int64_t)zl * N + tid] : 0.0;
+    const double gt = tid < N ? gv[(int64_t)zl * N + tid] : 0.0;
+    if (tid < kMaxN) x0[tid] = gt;
     double y = mul_t(x0);
     if (tid < kMaxN) x1[tid] = tid < N ? y : 0.0;
     y = mul_t(x1);
+    // One step of refinement, a + T (T (g - A a)): the reduction's and the poles' errors leave T T g
+    // off by a part of |g|, which is up to lambda_max times the amplitudes. Without it the increments at
+    // the observations were 0.85 to 222 times as far off as an FP64 eigensolve's (geometric means over
+    // 200 zones, 65 to 128 members, one dominant eigenvalue of 10^6 the worst), with it 0.02 to
+    // 0.73. 16,200 zones of 100 members: 0.9 ms of 101 (the reduction included).
+    {
+      const double a0 = tid < N ? y : 0.0;
+      if (tid < kMaxN) x0[tid] = a0;
+      y = mul_a(x0);
+      if (tid < kMaxN) x1[tid] = tid < N ? gt - y : 0.0;
+      y = mul_t(x1);
+      if (tid < kMaxN) x0[tid] = tid < N ? y : 0.0;
+      y = a0 + mul_t(x0);
+    }
     int nan_flag = 0;
     if (tid < N) {
       ampl[(int64_t)zl * N + tid] = y;
