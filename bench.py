@@ -230,8 +230,8 @@ def algorithmic_work(c, nobs, stage):
     """Operations of one launch of a stage (per-zone counts x zones with observations):
     gram: p N (N+1) + 2 p N   (lower-triangular HS^T diag(c) HS plus HS^T diag(c) d)
     eig:  17 to 64 members: the digit products of k_zone_isqrt_oz on the tensor cores, two
-          products (A Y, Y Z) of 34 digit pairs (levels 0..7) a residual, three residuals (two
-          Newton steps); else 9 N^3 (Householder tridiagonalisation + QR with vectors) +
+          products (A Y, Y Z) of 34 digit pairs (levels 0..7) a residual, two residuals (one a
+          Newton step, none after the last); else 9 N^3 (Householder tridiagonalisation + QR with vectors) +
           2 N^3 + 4 N^2 (T, ampl) in FP64
     update: 2 nz N^2 + 2 nz N (Sf T and Sf ampl)."""
     N = c.N
@@ -242,7 +242,7 @@ def algorithmic_work(c, nobs, stage):
         return float(np.sum(p * N * (N + 1) + 2 * p * N))
     if stage == "eig":
         if 17 <= N <= 64:
-            return float(act.sum() * 3 * 2 * 34 * 2.0 * N ** 3)
+            return float(act.sum() * 2 * 2 * 34 * 2.0 * N ** 3)
         return float(act.sum() * (11.0 * N ** 3 + 4.0 * N ** 2))
     return float(np.sum(2 * nz * N * N + 2 * nz * N))
 

@@ -94,7 +94,9 @@ extern "C" {
                                     eigensolve) and the update on the FP64 CUDA cores instead
                                     of the tensor cores (exact 8-bit slice products, used for
                                     N <= 64) and the eigenvector-free transform of 65 to 128
-                                    members; both give FP64-level results                  */
+                                    members; both give FP64-level results (on the tensor
+                                    cores an element of Sa is within 2^-54 of its row's
+                                    largest element of Sf times its column's of T)         */
 
 typedef struct {
   int64_t n;        /* state vector size                                        */

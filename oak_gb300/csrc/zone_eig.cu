@@ -1303,17 +1303,19 @@ cudaError_t zone_eig_fp64(int N, int32_t nzc, double* d_GT, const double* d_g,
                           const int32_t* d_nobs, int rotate, double* d_ampl, int32_t* d_status,
                           double* d_aux, double* d_Z, int32_t* d_work, cudaStream_t st,
                           int tc_products) {
-  // Newton from FP32 eigenpairs, padded to 64: 16,200 zones of 64 members 9.1 against 38.4 ms,
-  // 30: 6.4 against 9.7, 20: 5.7 against 6.4, 16: 5.4 against 5.3; 16 zones of 64 members 0.45
-  // against 1.97 ms. One zone is the global analysis: the Gram matrix of all observations has
-  // eigenvalues beyond FP32's reach, and the multisection kernel is made for it.
+  // Newton from FP32 eigenpairs, padded to 64: 16,200 zones of 64 members 8.6 against 38.4 ms,
+  // 30: 6.4 against 9.7, 20: 5.9 against 6.4, 16: 5.4 against 5.3. Of few zones a whole call takes, at
+  // 64 members, 1.25 against 1.26 ms (16 zones) and 1.27 against 2.07 (64); of 3 to 24 zones of 24
+  // to 60 members it is 1 to 13 % behind (0.94 against 0.83 for 4 of 48), but 10 to 30 times as exact.
+  // One zone is the global analysis: the Gram matrix of all observations has eigenvalues beyond
+  // FP32's reach, and the multisection kernel is made for it.
   constexpr int kNewtonMinN = 17;
   if (tc_products && N >= kNewtonMinN && N <= isqrt_oz_max_n() && nzc > 1)
     return zone_eig_newton(N, nzc, d_GT, d_g, d_nobs, rotate, d_ampl, d_status, d_aux, d_Z, d_work,
                            st);
-  // wider ensembles, without eigenvectors (the eigensolve in 16,200 zones of 65 members 38 against
-  // 47 ms, of 80 58 against 76, of 100 101 against 181, of 128 235 against 405; 160 zones of 100
-  // members 2.1 against 13.1 ms). One zone as above
+  // wider ensembles, without eigenvectors (the eigensolve in 16,200 zones of 65 members 39 against
+  // 47 ms, of 80 59 against 76, of 100 103 against 181, of 128 238 against 405; a call of 2 zones of
+  // 100 members 1.85 against 3.3 ms, of 151 1.9 against 9.2). One zone as above
   if (tc_products && N > isqrt_oz_max_n() && N <= sqrt64_max_n() && nzc > 1)
     return zone_eig_rational(N, nzc, d_GT, d_g, d_nobs, rotate, d_ampl, d_status, d_aux, d_Z,
                              d_work, st);

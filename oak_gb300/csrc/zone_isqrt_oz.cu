@@ -40,9 +40,10 @@
 // the next zone's G and V are copied in while a zone finishes. Every mbarrier wait is bounded
 // (ZST_TIMEOUT).
 //
-// Measured, 64,800 zones of 64 members: 18 ms (85,000 cycles a zone; a level product ~2,700 of
-// tensor time, its staging ~2,000 and its read ~2,900, a step's four products with V ~9,000:
-// bound by the latency of that chain with one zone in flight), and 14 ms for the FP32 stages.
+// Measured, 64,800 zones of 64 members: 20 ms (18 and 85,000 cycles a zone without the amplitudes'
+// refinement; a level product ~2,700 of tensor time, its staging ~2,000 and its read ~2,900, a
+// step's four products with V ~9,000: bound by the latency of that chain with one zone in flight),
+// and 13 ms for the FP32 stages.
 // The FP64 eigensolve and its tensor-core transform took 146 ms (FP64 pipe at 85-90 %). Errors
 // against long double on a zone: 1e-15, where an FP64 eigensolve has 1e-14 to 1e-13.
 #include <cuda_fp16.h>

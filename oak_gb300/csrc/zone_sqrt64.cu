@@ -26,7 +26,7 @@
 // reflectors (the products F v of all columns, the update of the lower triangle), an eighth the
 // poles. The eigenvector path it replaces spent 2 N^3 on U and U f(L) U^T, besides the
 // orthogonalisation: 16,200 zones of 100 members 152 ms (eigenvalues 11, inverse iteration 9, U and
-// T 132) against 66.5 ms here. Per zone, of about 1.3 million cycles: 29% F v, 27% the update, 19% the
+// T 132) against 67.4 ms here. Per zone, of about 1.3 million cycles: 29% F v, 27% the update, 19% the
 // poles' recurrences (their warp shares its partition's pipe with the other block), 6% columns of F.
 // Layout: one zone a block of 256 threads, F's lower triangle in shared memory with an odd row
 // stride (rows and columns are read without conflicts), two blocks an SM up to about 100 members, so
